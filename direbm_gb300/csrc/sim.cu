@@ -73,8 +73,13 @@ __global__ void __launch_bounds__(256) k_collide(const __grid_constant__ Args<Q,
       } else {
         collide_moment_dev<Q, D>(A.a.rho[m], dv, (float)I.tau, A.L);
       }
+      float big = fabsf(A.a.rho[m]);  // NaN or infinite when the density or some f* is
 #pragma unroll
-      for (int k = 0; k < Q; ++k) A.a.dev[(int64_t)k * A.mcap + m] = dv[k];
+      for (int k = 0; k < Q; ++k) {
+        A.a.dev[(int64_t)k * A.mcap + m] = dv[k];
+        big = __fadd_rn(big, fabsf(dv[k]));
+      }
+      if (A.odd_f && !(A.a.rho[m] >= 0.f && big < 3.4e38f)) *A.odd_f = 1;
       if (A.want_wexp) {
         const float rho = A.a.rho[m];
 #pragma unroll
@@ -837,11 +842,12 @@ __global__ void __launch_bounds__(256, gather_min_blocks<P>()) k_gather(const __
 }
 
 template <int Q, int D, class P>
-__global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D, P> A) {
+__global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D, P> A, int only_gaps) {
   using real = typename P::real;
   const uint32_t Pn = *A.d_P;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < Pn; j += gridDim.x * blockDim.x) {
     const uint32_t em = A.emask[j];
+    if (only_gaps && !em) continue;  // emitted by the gather
     const uint32_t G = A.b.cell[j];
     const int b = find_instance(A.inst_base, A.n_inst, G);
     const InstK I = A.inst[b];
@@ -1295,6 +1301,7 @@ struct SimImpl : SimBase {
   size_t sm_gather_s = 0;
   // dense-stencil kernels (k_*_ds, shared memory = the dense layout) and the list of tiles they
   // defer to the row-segment code: d_fb[0..2] the per-stage counts, d_fb + 4 the tile indices
+  bool near_ok = false;         // their NEAR variants apply (dx = cell, D2Q9, 1 <= R < 2)
   size_t sm_ds[3] = {0, 0, 0};  // thin+refine, weights, gather
   int pgrid_ds[3] = {1, 1, 1};
   int* d_fb = nullptr;
@@ -1629,9 +1636,15 @@ struct SimImpl : SimBase {
     if (shift_ok) {
       geo_s.cap_gather = pick_cap(3, mcells, budget);
       sm_gather_s = smem_for(3, geo_s.cap_gather);
-      sm_ds[0] = ds_bytes_refine(Q, mcells);
-      sm_ds[1] = ds_bytes_weights(ccells);
-      sm_ds[2] = ds_bytes_gather(Q, mcells);
+      sm_ds[0] = DenseLayoutOf<Q, 0, 0>::make(geo).total;
+      sm_ds[1] = DenseLayoutOf<Q, 1, 0>::make(geo).total;
+      sm_ds[2] = DenseLayoutOf<Q, 2, 0>::make(geo).total;
+      // the NEAR dense kernels: displacements of exactly one cell in D2Q9's order, and R >= 1, so that
+      // a 6 x 6 block around any reference point lies in the staged region, which has 3 cells of halo
+      near_ok = Q == 9 && R >= 1.0;
+      for (const Halo& h : {m, c}) near_ok = near_ok && h.xl == -3 && h.xh == 3 && h.yl == -3 && h.yh == 3;
+      for (int k = 0; k < Q && near_ok; ++k)
+        near_ok = LH.c[k][0] * desc.dx / desc.cell == d2q9_cx(k) && LH.c[k][1] * desc.dx / desc.cell == d2q9_cy(k);
     }
     std::vector<Tile2> tiles;
     for (int i = 0; i < (int)inst_h.size(); ++i)
@@ -1681,8 +1694,12 @@ struct SimImpl : SimBase {
           int nbw = 1;
           DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbw, k_weights_t<Q, P, true>, 256, sm_weights));
           pgrid_ws = std::max(1, std::min(ntiles, std::max(nbw, 1) * sm_count()));
-          const void* kds[3] = {(const void*)k_thin_refine_ds<Q>, (const void*)k_weights_ds<Q>,
-                                (const void*)k_gather_ds<Q>};
+          const void* kds[3];
+          with_near([&](auto tx) {
+            kds[0] = (const void*)k_thin_refine_ds<Q, tx.value>;
+            kds[1] = (const void*)k_weights_ds<Q, tx.value>;
+            kds[2] = (const void*)k_gather_ds<Q, tx.value>;
+          });
           for (int i = 0; i < 3; ++i) {
             DBM_CUDA(cudaFuncSetAttribute(kds[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
             int nbd = 1;
@@ -1844,6 +1861,21 @@ struct SimImpl : SimBase {
   // the untiled window kernels.
   bool tiled_path() const { return D == 2 && tiled && use_tiles && !args.any_obstacle && args.kappa_soft == 0; }
 
+  // fn(integral constant): the tile width for the NEAR dense kernels, 0 where they do not apply.
+  template <class Fn>
+  void with_near(Fn&& fn) {
+    if constexpr (Q == 9) {
+      if (near_ok) {
+        if (geo.tx == 8) return fn(std::integral_constant<int, 8>{});
+        if (geo.tx == 16) return fn(std::integral_constant<int, 16>{});
+        if (geo.tx == 32) return fn(std::integral_constant<int, 32>{});
+        if (geo.tx == 64) return fn(std::integral_constant<int, 64>{});
+        return fn(std::integral_constant<int, 128>{});
+      }
+    }
+    fn(std::integral_constant<int, 0>{});
+  }
+
   int launch_step(cudaStream_t s, int upto) {
     bind();
     Args<Q, D, P>& A = args;
@@ -1857,6 +1889,8 @@ struct SimImpl : SimBase {
       return DBM_ERR_STATE;
     }
     A.want_wexp = untiled ? 1 : 0;
+    A.odd_f = d_fb ? d_fb + 3 : nullptr;
+    if (d_fb) DBM_CUDA(cudaMemsetAsync(d_fb, 0, 4 * sizeof(int), s));  // fallback counts of the three stages, odd_f
     k_collide<Q, D, P><<<gm, 256, 0, s>>>(A);
     DBM_LAUNCH_CHECK();
     if (untiled) {
@@ -1870,11 +1904,12 @@ struct SimImpl : SimBase {
         bool shifted = false;
         if constexpr (std::is_same<P, PF32>::value) {
           if (shift_ok && use_shift && use_dense) {
-            DBM_CUDA(cudaMemsetAsync(d_fb, 0, 3 * sizeof(int), s));  // the three stages' fallback counts
-            k_thin_refine_ds<Q><<<use_persistent ? pgrid_ds[0] : ntiles, 256, sm_ds[0], s>>>(A, d_tiles, geo, ntiles,
-                                                                                            d_fb + 4, d_fb + 0);
+            const int grid = use_persistent ? pgrid_ds[0] : ntiles;
+            with_near([&](auto tx) {
+              k_thin_refine_ds<Q, tx.value><<<grid, 256, sm_ds[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
+            });
             DBM_LAUNCH_CHECK();
-            k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0);
+            k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
             shifted = true;
           } else if (shift_ok && use_shift) {
             k_thin_refine_t<Q, P, true><<<use_persistent ? pgrid_rs : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo,
@@ -1932,10 +1967,12 @@ struct SimImpl : SimBase {
         bool shifted = false;
         if constexpr (std::is_same<P, PF32>::value) {
           if (shift_ok && use_shift && use_dense) {
-            k_weights_ds<Q><<<use_persistent ? pgrid_ds[1] : ntiles, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles,
-                                                                                        d_fb + 4, d_fb + 1);
+            const int grid = use_persistent ? pgrid_ds[1] : ntiles;
+            with_near([&](auto tx) {
+              k_weights_ds<Q, tx.value><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+            });
             DBM_LAUNCH_CHECK();
-            k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1);
+            k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
             shifted = true;
           } else if (shift_ok && use_shift) {
             k_weights_t<Q, P, true><<<use_persistent ? pgrid_ws : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo,
@@ -1954,16 +1991,23 @@ struct SimImpl : SimBase {
     DBM_LAUNCH_CHECK();
     mark(4, s);
     if (upto <= 4) return DBM_OK;
-    DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
+    // the dense gather writes every control point's empty mask and, unless the step keeps its
+    // intermediates, emits the points without an empty direction itself
+    bool dense = false;
+    if constexpr (D == 2 && std::is_same<P, PF32>::value) dense = tiled_path() && shift_ok && use_shift && use_dense;
+    const int fuse = dense && !A.write_trace ? 1 : 0;
+    if (!dense) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (D == 2) {
       if (tiled_path()) {
         bool shifted = false;
         if constexpr (std::is_same<P, PF32>::value) {
           if (shift_ok && use_shift && use_dense) {
-            k_gather_ds<Q><<<use_persistent ? pgrid_ds[2] : ntiles, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles,
-                                                                                       d_fb + 4, d_fb + 2);
+            const int grid = use_persistent ? pgrid_ds[2] : ntiles;
+            with_near([&](auto tx) {
+              k_gather_ds<Q, tx.value><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + 4, d_fb + 2, fuse);
+            });
             DBM_LAUNCH_CHECK();
-            k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2);
+            k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2, fuse);
             shifted = true;
           } else if (shift_ok && use_shift) {
             k_gather_ts<Q><<<use_persistent ? pgrid_s : ntiles, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, ntiles);
@@ -1981,7 +2025,7 @@ struct SimImpl : SimBase {
     DBM_LAUNCH_CHECK();
     mark(5, s);
     if (upto <= 5) return DBM_OK;
-    k_emit<Q, D, P><<<gc, 256, 0, s>>>(A);
+    k_emit<Q, D, P><<<gc, 256, 0, s>>>(A, fuse);
     DBM_LAUNCH_CHECK();
     mark(6, s);
     return DBM_OK;

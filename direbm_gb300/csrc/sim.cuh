@@ -129,6 +129,7 @@ struct Args {
   int any_obstacle;
   uint32_t* status;
   uint32_t* d_P;
+  int* odd_f;      // (dense kernels) set by the collision: a density is negative or an f* not finite
   int write_trace;
 };
 
