@@ -1224,7 +1224,7 @@ __global__ void __launch_bounds__(256) k_conservation(const __grid_constant__ Ar
 
 }  // namespace dbm
 
-#include "sim_dense.cuh"
+#include "sim_grid.cuh"
 
 namespace dbm {
 
@@ -1303,6 +1303,10 @@ struct SimImpl : SimBase {
   // defer to the row-segment code: d_fb[0..2] the per-stage counts, d_fb + 4 the tile indices
   bool near_ok = false;         // their NEAR variants apply (dx = cell, D2Q9, 1 <= R < 2)
   size_t sm_ds[3] = {0, 0, 0};  // thin+refine, weights, gather
+  // grid kernels (k_*_grid): window width W in cells they are compiled for, 0 where they do not apply
+  int grid_w = 0;
+  size_t sm_grid[3] = {0, 0, 0};
+  int pgrid_grid[3] = {1, 1, 1};
   int pgrid_ds[3] = {1, 1, 1};
   int* d_fb = nullptr;
   int use_persistent = 0;
@@ -1646,6 +1650,18 @@ struct SimImpl : SimBase {
       for (int k = 0; k < Q && near_ok; ++k)
         near_ok = LH.c[k][0] * desc.dx / desc.cell == d2q9_cx(k) && LH.c[k][1] * desc.dx / desc.cell == d2q9_cy(k);
     }
+    // grid kernels: FP32, displacements or radius that the dense kernels do not take, a window of
+    // ceil(2 R) + 1 cells of a compiled width (4: 1 < R <= 1.5, 9: 3.5 < R <= 4, the radii in use)
+    grid_w = 0;
+    if (std::is_same<P, PF32>::value && !shift_ok && (Q == 7 || Q == 9)) {
+      const int w = (int)std::ceil(2 * R - 1e-3) + 1;
+      if (w == 4 || w == 9) grid_w = w;
+      for (int i = 0; i < 3 && grid_w; ++i) {
+        const GridLayout L = grid_layout(Q, i, geo);
+        sm_grid[i] = (size_t)L.total;
+        if (sm_grid[i] > 200 * 1024 || L.rw >= 4096 || L.rh >= 2048) grid_w = 0;  // the list's keys hold 12 + 11 bits
+      }
+    }
     std::vector<Tile2> tiles;
     for (int i = 0; i < (int)inst_h.size(); ++i)
       for (int y0 = 0; y0 < inst_h[i].dims[1]; y0 += geo.ty)
@@ -1661,7 +1677,7 @@ struct SimImpl : SimBase {
       release(d_fb);
       d_fb = nullptr;
     }
-    if (shift_ok) {
+    if (shift_ok || grid_w) {
       DBM_TRY(alloc(&d_fb, (int64_t)ntiles + 4));
       DBM_CUDA(cudaMemset(d_fb, 0, ((size_t)ntiles + 4) * sizeof(int)));
     }
@@ -1678,6 +1694,24 @@ struct SimImpl : SimBase {
       DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[2], k_gather_t<Q, P>, 256, sm_gather));
       for (int i = 0; i < 3; ++i) pgrid[i] = std::max(1, std::min(ntiles, std::max(nb[i], 1) * sm_count()));
       if constexpr (std::is_same<P, PF32>::value) {
+        if (grid_w) {
+          const void* kg[3];
+          with_grid([&](auto w) {
+            kg[0] = (const void*)k_thin_refine_grid<Q, w.value>;
+            kg[1] = (const void*)k_weights_grid<Q, w.value>;
+            kg[2] = (const void*)k_gather_grid<Q, w.value>;
+          });
+          const void* kf[3] = {(const void*)k_grid_fallback<Q, 0>, (const void*)k_grid_fallback<Q, 1>,
+                               (const void*)k_grid_fallback<Q, 2>};
+          const size_t sf[3] = {sm_refine, sm_weights, sm_gather};
+          for (int i = 0; i < 3; ++i) {
+            DBM_CUDA(cudaFuncSetAttribute(kg[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_grid[i]));
+            DBM_CUDA(cudaFuncSetAttribute(kf[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf[i]));
+            int nbd = 1;
+            DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kg[i], 256, sm_grid[i]));
+            pgrid_grid[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
+          }
+        }
         if (shift_ok) {
           DBM_CUDA(cudaFuncSetAttribute((const void*)k_gather_ts<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sm_gather_s));
@@ -1876,6 +1910,14 @@ struct SimImpl : SimBase {
     fn(std::integral_constant<int, 0>{});
   }
 
+  // fn(integral constant): the window width of the grid kernels (grid_w != 0).
+  template <class Fn>
+  void with_grid(Fn&& fn) {
+    if (grid_w == 4) fn(std::integral_constant<int, 4>{});
+    else fn(std::integral_constant<int, 9>{});
+  }
+  bool grid_path() const { return grid_w != 0 && use_dense && tiled_path(); }
+
   int launch_step(cudaStream_t s, int upto) {
     bind();
     Args<Q, D, P>& A = args;
@@ -1910,6 +1952,14 @@ struct SimImpl : SimBase {
             });
             DBM_LAUNCH_CHECK();
             k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
+            shifted = true;
+          } else if (grid_path()) {
+            const int grid = use_persistent ? pgrid_grid[0] : ntiles;
+            with_grid([&](auto w) {
+              k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
+            });
+            DBM_LAUNCH_CHECK();
+            k_grid_fallback<Q, 0><<<pgrid[0], 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
             shifted = true;
           } else if (shift_ok && use_shift) {
             k_thin_refine_t<Q, P, true><<<use_persistent ? pgrid_rs : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo,
@@ -1974,6 +2024,14 @@ struct SimImpl : SimBase {
             DBM_LAUNCH_CHECK();
             k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
             shifted = true;
+          } else if (grid_path()) {
+            const int grid = use_persistent ? pgrid_grid[1] : ntiles;
+            with_grid([&](auto w) {
+              k_weights_grid<Q, w.value><<<grid, 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+            });
+            DBM_LAUNCH_CHECK();
+            k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
+            shifted = true;
           } else if (shift_ok && use_shift) {
             k_weights_t<Q, P, true><<<use_persistent ? pgrid_ws : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo,
                                                                                                ntiles);
@@ -1994,7 +2052,7 @@ struct SimImpl : SimBase {
     // the dense gather writes every control point's empty mask and, unless the step keeps its
     // intermediates, emits the points without an empty direction itself
     bool dense = false;
-    if constexpr (D == 2 && std::is_same<P, PF32>::value) dense = tiled_path() && shift_ok && use_shift && use_dense;
+    if constexpr (D == 2 && std::is_same<P, PF32>::value) dense = (tiled_path() && shift_ok && use_shift && use_dense) || grid_path();
     const int fuse = dense && !A.write_trace ? 1 : 0;
     if (!dense) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (D == 2) {
@@ -2008,6 +2066,14 @@ struct SimImpl : SimBase {
             });
             DBM_LAUNCH_CHECK();
             k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2, fuse);
+            shifted = true;
+          } else if (grid_path()) {
+            const int grid = use_persistent ? pgrid_grid[2] : ntiles;
+            with_grid([&](auto w) {
+              k_gather_grid<Q, w.value><<<grid, 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 2, fuse);
+            });
+            DBM_LAUNCH_CHECK();
+            k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 2, fuse);
             shifted = true;
           } else if (shift_ok && use_shift) {
             k_gather_ts<Q><<<use_persistent ? pgrid_s : ntiles, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, ntiles);

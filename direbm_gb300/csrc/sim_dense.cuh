@@ -334,6 +334,54 @@ struct WeightSum2 {
 // ---- thinning + refine --------------------------------------------------------------------------
 // Float planes: exp(f*_k) of each item.
 
+// The refined control point of cell F: the move for kappa > kappa_hard, its cell and offsets.
+template <int Q>
+__device__ __forceinline__ void refine_store(const Args<Q, 2, PF32>& A, const InstK& I, uint32_t F, int Fx, int Fy,
+                                             uint32_t cnt, uint32_t mask, const float (&cen)[2], float swf, float2 sx) {
+  const int kappa = __popc(mask);
+  float np[2];
+  if (kappa <= A.kappa_hard) {
+    np[0] = cen[0];
+    np[1] = cen[1];
+  } else {
+    np[0] = cen[0] + sx.x / swf;
+    np[1] = cen[1] + sx.y / swf;
+  }
+  bool finite = true;
+#pragma unroll
+  for (int a = 0; a < 2; ++a) finite &= isfinite(np[a]) && fabsf(np[a]) < 64.f;
+  if (!finite) {
+    atomicOr(A.status, ST_NONFINITE);
+    np[0] = cen[0];
+    np[1] = cen[1];
+  }
+  int sh[2];
+  float off[2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    const float fl = floorf(np[a]);
+    sh[a] = (int)fl;
+    off[a] = np[a] - fl;
+    if (off[a] >= 1.f) {
+      off[a] = 0.f;
+      sh[a] += 1;
+    }
+  }
+  uint32_t Gc;
+  const bool inside = cell_at<2>(I, Fx + sh[0], Fy + sh[1], 0, &Gc);
+  if (!inside) atomicOr(A.status, ST_OUT_OF_BOX);
+  A.occ[F] = inside ? 1u : 0u;
+  A.fkey[F] = inside ? Gc : 0xffffffffu;
+  A.foff[F] = off[0];
+  A.foff[(int64_t)A.ncells + F] = off[1];
+  if (A.write_trace) {
+    A.tcnt[F] = cnt;
+    A.mask[F] = mask;
+    A.cen[F] = cen[0];
+    A.cen[(int64_t)A.ncells + F] = cen[1];
+  }
+}
+
 template <int Q, int TX>
 __device__ __forceinline__ bool thin_refine_ds_tile(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
                                                     const TileGeo& G, unsigned char* smem) {
@@ -497,48 +545,7 @@ __device__ __forceinline__ bool thin_refine_ds_tile(const Args<Q, 2, PF32>& A, c
       if (dmin <= A.R2) mask |= 1u << k;
     }
   }
-  const int kappa = __popc(mask);
-  float np[2];
-  if (kappa <= A.kappa_hard) {
-    np[0] = cen[0];
-    np[1] = cen[1];
-  } else {
-    np[0] = cen[0] + sx.x / swf;
-    np[1] = cen[1] + sx.y / swf;
-  }
-  bool finite = true;
-#pragma unroll
-  for (int a = 0; a < 2; ++a) finite &= isfinite(np[a]) && fabsf(np[a]) < 64.f;
-  if (!finite) {
-    atomicOr(A.status, ST_NONFINITE);
-    np[0] = cen[0];
-    np[1] = cen[1];
-  }
-  int sh[2];
-  float off[2];
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const float fl = floorf(np[a]);
-    sh[a] = (int)fl;
-    off[a] = np[a] - fl;
-    if (off[a] >= 1.f) {
-      off[a] = 0.f;
-      sh[a] += 1;
-    }
-  }
-  uint32_t Gc;
-  const bool inside = cell_at<2>(I, Fx + sh[0], Fy + sh[1], 0, &Gc);
-  if (!inside) atomicOr(A.status, ST_OUT_OF_BOX);
-  A.occ[F] = inside ? 1u : 0u;
-  A.fkey[F] = inside ? Gc : 0xffffffffu;
-  A.foff[F] = off[0];
-  A.foff[(int64_t)A.ncells + F] = off[1];
-  if (A.write_trace) {
-    A.tcnt[F] = cnt;
-    A.mask[F] = mask;
-    A.cen[F] = cen[0];
-    A.cen[(int64_t)A.ncells + F] = cen[1];
-  }
+  refine_store<Q>(A, I, F, Fx, Fy, cnt, mask, cen, swf, sx);
   return true;
 }
 
@@ -1007,6 +1014,27 @@ __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_GATHER) k_gather_ds(const _
   }
 }
 
+// A deferred tile's gather: clears its control points' empty masks, runs `gather`, and with fuse
+// emits the points that end up without an empty direction.
+template <int Q, class Fn>
+__device__ __forceinline__ void gather_fallback(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
+                                                const TileGeo& G, bool fuse, Fn&& gather) {
+  const int lx = threadIdx.x % G.tx, ly = threadIdx.x / G.tx;
+  uint32_t jb = 0, je = 0;  // this thread's cell's control points
+  if (ly < G.ty && T.x0 + lx < I.dims[0] && T.y0 + ly < I.dims[1]) {
+    const uint32_t g = I.base + (uint32_t)(T.x0 + lx) + (uint32_t)I.dims[0] * (uint32_t)(T.y0 + ly);
+    jb = A.b.start[g];
+    je = A.b.start[g + 1];
+  }
+  for (uint32_t j = jb; j < je; ++j) A.emask[j] = 0u;
+  __syncthreads();
+  gather();
+  __syncthreads();
+  if (fuse)
+    for (uint32_t j = jb; j < je; ++j)
+      if (__ldcg(A.emask + j) == 0u) emit_from_cpf<Q>(A, (int)j);
+}
+
 // Row-segment passes over the deferred tiles (persistent grid; nothing to do when the list is
 // empty).  STAGE: 0 thin + refine, 1 weights, 2 gather (which first clears its control points' empty
 // masks and, with fuse, emits those that end up without an empty direction).
@@ -1025,20 +1053,7 @@ __global__ void __launch_bounds__(256) k_dense_fallback(const __grid_constant__ 
     } else if constexpr (STAGE == 1) {
       weights_tile<Q, PF32, true>(A, T, I, G, smem);
     } else {
-      const int lx = threadIdx.x % G.tx, ly = threadIdx.x / G.tx;
-      uint32_t jb = 0, je = 0;  // this thread's cell's control points
-      if (ly < G.ty && T.x0 + lx < I.dims[0] && T.y0 + ly < I.dims[1]) {
-        const uint32_t g = I.base + (uint32_t)(T.x0 + lx) + (uint32_t)I.dims[0] * (uint32_t)(T.y0 + ly);
-        jb = A.b.start[g];
-        je = A.b.start[g + 1];
-      }
-      for (uint32_t j = jb; j < je; ++j) A.emask[j] = 0u;
-      __syncthreads();
-      gather_ts_tile<Q>(A, T, I, G, smem);
-      __syncthreads();
-      if (fuse)
-        for (uint32_t j = jb; j < je; ++j)
-          if (__ldcg(A.emask + j) == 0u) emit_from_cpf<Q>(A, (int)j);
+      gather_fallback<Q>(A, T, I, G, fuse != 0, [&] { gather_ts_tile<Q>(A, T, I, G, smem); });
     }
     __syncthreads();
   }

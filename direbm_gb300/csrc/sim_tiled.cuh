@@ -1350,15 +1350,12 @@ __global__ void __launch_bounds__(256) k_gather_ts(const __grid_constant__ Args<
   }
 }
 
+// One tile of the gather, staged through `smem`.
 template <int Q, class P>
-__global__ void __launch_bounds__(256) k_gather_t(const __grid_constant__ Args<Q, 2, P> A,
-                                                 const Tile2* __restrict__ tiles, const TileGeo G, int ntiles) {
+__device__ __forceinline__ void gather_tile(const Args<Q, 2, P>& A, const Tile2& T, const InstK& I, const TileGeo& G,
+                                            unsigned char* smem) {
   using real = typename P::real;
   constexpr bool F64 = std::is_same<P, PF64>::value;
-  extern __shared__ __align__(16) unsigned char smem[];
-  for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
-  const Tile2 T = tiles[tb];
-  const InstK I = A.inst[T.inst];
   const int rw = G.tx + G.mom.xh - G.mom.xl, rh = G.ty + G.mom.yh - G.mom.yl;
   const int cap = G.cap_gather, cap_t = G.cap_tile;
   unsigned char* p = smem;
@@ -1386,7 +1383,17 @@ __global__ void __launch_bounds__(256) k_gather_t(const __grid_constant__ Args<Q
   else
     gather_body<Q, P, false>(A, I, T, G, rw, rh, s_beg, s_end, s_gi, nullptr, s_rho, s_kv, 0, s_tr, s_ij, s_bx, s_by,
                              s_cpos);
-  __syncthreads();
+}
+
+template <int Q, class P>
+__global__ void __launch_bounds__(256) k_gather_t(const __grid_constant__ Args<Q, 2, P> A,
+                                                 const Tile2* __restrict__ tiles, const TileGeo G, int ntiles) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
+    const Tile2 T = tiles[tb];
+    const InstK I = A.inst[T.inst];
+    gather_tile<Q, P>(A, T, I, G, smem);
+    __syncthreads();
   }
 }
 
