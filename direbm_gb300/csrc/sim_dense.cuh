@@ -460,6 +460,7 @@ __device__ __forceinline__ bool thin_refine_ds_tile(const Args<Q, 2, PF32>& A, c
   }
   if (cnt == 0) {
     A.occ[F] = 0u;
+    A.fkey[F] = 0xffffffffu;  // read by the placement's neighbourhood search
     if (A.write_trace) {
       A.tcnt[F] = 0u;
       A.mask[F] = 0u;
@@ -771,8 +772,8 @@ __device__ __forceinline__ DF gather_ds_unit(const Args<Q, 2, PF32>& A, const SM
 
 // Control point j with all nine sums known and no empty direction: the next moment's density and
 // deviations (k_emit's arithmetic).
-template <int Q>
-__device__ __forceinline__ void emit_full(const Args<Q, 2, PF32>& A, int j, const DF (&F)[Q]) {
+template <int Q, int D>
+__device__ __forceinline__ void emit_full(const Args<Q, D, PF32>& A, int j, const DF (&F)[Q]) {
   DF rho = {0.f, 0.f};
 #pragma unroll
   for (int k = 0; k < Q; ++k) rho = df_add(rho, F[k]);
@@ -781,8 +782,8 @@ __device__ __forceinline__ void emit_full(const Args<Q, 2, PF32>& A, int j, cons
   for (int k = 0; k < Q; ++k)
     A.b.dev[(int64_t)k * A.ccap + j] = df_float(df_add(F[k], df_neg(df_mul(DF{A.L.wf[k], A.L.wlo[k]}, rho))));
 }
-template <int Q>
-__device__ __forceinline__ void emit_from_cpf(const Args<Q, 2, PF32>& A, int j) {
+template <int Q, int D>
+__device__ __forceinline__ void emit_from_cpf(const Args<Q, D, PF32>& A, int j) {
   DF F[Q];
 #pragma unroll
   for (int k = 0; k < Q; ++k) F[k] = DF{A.cpfhi[(int64_t)k * A.ccap + j], A.cpflo[(int64_t)k * A.ccap + j]};

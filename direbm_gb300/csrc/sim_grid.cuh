@@ -261,6 +261,7 @@ __device__ __forceinline__ bool thin_refine_grid_tile(const Args<Q, 2, PF32>& A,
   }
   if (cnt == 0) {
     A.occ[F] = 0u;
+    A.fkey[F] = 0xffffffffu;  // read by the placement's neighbourhood search
     if (A.write_trace) {
       A.tcnt[F] = 0u;
       A.mask[F] = 0u;

@@ -302,6 +302,7 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
   if (!valid) return;
   if (!occupied) {
     A.occ[F] = 0u;
+    A.fkey[F] = 0xffffffffu;  // read by the placement's neighbourhood search
     if (A.write_trace) {
       A.tcnt[F] = 0u;
       A.mask[F] = 0u;
@@ -506,6 +507,7 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
   }
   if (cnt == 0) {
     A.occ[F] = 0u;
+    A.fkey[F] = 0xffffffffu;  // read by the placement's neighbourhood search
     if (A.write_trace) {
       A.tcnt[F] = 0u;
       A.mask[F] = 0u;
