@@ -1224,7 +1224,7 @@ __global__ void __launch_bounds__(256) k_conservation(const __grid_constant__ Ar
 
 }  // namespace dbm
 
-#include "sim_grid.cuh"
+#include "sim_grid3.cuh"
 
 namespace dbm {
 
@@ -1309,6 +1309,13 @@ struct SimImpl : SimBase {
   int pgrid_grid[3] = {1, 1, 1};
   int pgrid_ds[3] = {1, 1, 1};
   int* d_fb = nullptr;
+  // 3D grid kernels (k_brick3): bricks of 8^3 cells away from obstacles, the other bricks (8 x 8 x 4, for
+  // the untiled kernels), and per stage the bricks they defer (d_fb3[0..2] counts, [3] odd_f, + 4 list)
+  bool brick3_ok = false;
+  bool bricks3_stale = true;
+  Brick *d_bricks3 = nullptr, *d_near3 = nullptr;
+  int nbricks3 = 0, nnear3 = 0;
+  int* d_fb3 = nullptr;
   int use_persistent = 0;
   TileGeo geo{};
   size_t sm_refine = 0, sm_weights = 0, sm_gather = 0;
@@ -1494,11 +1501,115 @@ struct SimImpl : SimBase {
     DBM_CUDA(cudaMemset(A.status, 0, 4));
     DBM_CUDA(cudaMemset(A.d_P, 0, 4));
     if constexpr (D == 2) DBM_TRY(init_tiles(LH, R));
+    if constexpr (D == 3 && std::is_same<P, PF32>::value) DBM_TRY(init_brick3(LH, R));
     DBM_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
     DBM_CUDA(cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming));
     DBM_CUDA(cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming));
     DBM_TRY(set_brick(D == 3 ? 8 : 16));  // 8 x 8 x 4 in 3D, 16 x 16 in 2D
     if (!tiled) DBM_TRY(ensure_untiled());  // 3D: always the untiled window kernels
+    return DBM_OK;
+  }
+
+  // The 3D grid kernels serve windows of ceil(2 R) + 1 = 4 cells (1 < R <= 1.5, the radii in use) whose
+  // region lies within kHalo3 cells of a brick.
+  int init_brick3(const LatHost& LH, double R) {
+    if constexpr (D == 3 && std::is_same<P, PF32>::value) {
+      if ((int)std::ceil(2 * R - 1e-3) + 1 != 4) return DBM_OK;
+      const double tiny = 2e-4;
+      for (int k = 0; k < Q; ++k)
+        for (int a = 0; a < 3; ++a) {
+          const double cd = std::fabs(LH.c[k][a] * desc.dx / desc.cell) * (1 + 1e-6);
+          if (std::floor(-cd - R - tiny) < -kHalo3 || std::floor(1 + cd + R + tiny) > kHalo3) return DBM_OK;
+        }
+      const void* k3[3] = {(const void*)k_brick3<Q, 0>, (const void*)k_brick3<Q, 1>, (const void*)k_brick3<Q, 2>};
+      for (int i = 0; i < 3; ++i)
+        DBM_CUDA(cudaFuncSetAttribute(k3[i], cudaFuncAttributeMaxDynamicSharedMemorySize, grid3_layout(i).total));
+      brick3_ok = true;
+    }
+    return DBM_OK;
+  }
+
+  // The brick lists of the 3D grid kernels: a brick belongs to the untiled kernels when a point of it
+  // could meet a bounced component, or a moment of its region be one (the obstacle's reach, set_obstacle).
+  int make_bricks3() {
+    if constexpr (D == 3 && std::is_same<P, PF32>::value) {
+      if (!brick3_ok || !bricks3_stale) return DBM_OK;
+      std::vector<Brick> far, near;
+      for (int i = 0; i < (int)inst_h.size(); ++i) {
+        const InstK& I = inst_h[i];
+        for (int z0 = 0; z0 < I.dims[2]; z0 += kBrick3)
+          for (int y0 = 0; y0 < I.dims[1]; y0 += kBrick3)
+            for (int x0 = 0; x0 < I.dims[0]; x0 += kBrick3) {
+              bool clear = true;
+              if (I.has_obs) {
+                const int b0[3] = {x0, y0, z0};
+                double d2 = 0;
+                for (int a = 0; a < 3; ++a) {  // distance of the center from the brick with its halo
+                  const double lo = b0[a] - kHalo3 - 1, hi = b0[a] + kBrick3 + kHalo3 + 1;
+                  const double e = std::max({lo - I.obs_c[a], I.obs_c[a] - hi, 0.0});
+                  d2 += e * e;
+                }
+                clear = d2 > std::max((double)I.reach2, (double)I.near2);
+              }
+              if (clear) {
+                far.push_back({i, x0, y0, z0});
+              } else {
+                near.push_back({i, x0, y0, z0});
+                if (z0 + kBrick3 / 2 < I.dims[2]) near.push_back({i, x0, y0, z0 + kBrick3 / 2});
+              }
+            }
+      }
+      DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the old lists
+      release(d_bricks3);
+      release(d_near3);
+      release(d_fb3);
+      d_bricks3 = d_near3 = nullptr;
+      d_fb3 = nullptr;
+      DBM_TRY(alloc(&d_bricks3, (int64_t)far.size()));
+      DBM_TRY(alloc(&d_near3, (int64_t)near.size()));
+      DBM_TRY(alloc(&d_fb3, (int64_t)far.size() + 4));
+      DBM_CUDA(cudaMemcpy(d_bricks3, far.data(), sizeof(Brick) * far.size(), cudaMemcpyHostToDevice));
+      DBM_CUDA(cudaMemcpy(d_near3, near.data(), sizeof(Brick) * near.size(), cudaMemcpyHostToDevice));
+      nbricks3 = (int)far.size();
+      nnear3 = (int)near.size();
+      bricks3_stale = false;
+      invalidate_graphs();  // captured launches hold the lists
+    }
+    return DBM_OK;
+  }
+  bool brick3_path() const { return D == 3 && brick3_ok && use_tiles && use_dense && args.kappa_soft == 0; }
+
+  // Stage `STAGE` of the 3D grid kernels: the clear bricks, those they deferred, and the near ones.
+  template <int STAGE>
+  int launch_brick3(Args<Q, D, P>& A, int fuse, cudaStream_t s) {
+    if constexpr (D == 3 && std::is_same<P, PF32>::value) {
+      const BrickGeo half{kBrick3, kBrick3, kBrick3 / 2};
+      if (nbricks3 > 0) {
+        constexpr int smem = grid3_layout(STAGE).total;
+        k_brick3<Q, STAGE><<<nbricks3, kThreads3, smem, s>>>(A, d_bricks3, nbricks3, d_fb3 + 4, d_fb3 + STAGE, fuse);
+        DBM_LAUNCH_CHECK();
+        const unsigned gf = (unsigned)std::min<int64_t>((int64_t)nbricks3 * (STAGE == 0 ? 2 : 2 * Q), sm_count() * 6);
+        k_brick3_fallback<Q, STAGE><<<gf, 256, 0, s>>>(A, d_bricks3, d_fb3 + 4, d_fb3 + STAGE);
+        DBM_LAUNCH_CHECK();
+      }
+      if (nnear3 > 0) {
+        if constexpr (STAGE == 0) k_thin_refine<Q, D, P><<<nnear3, 256, 0, s>>>(A, d_near3, nnear3, half);
+        else if constexpr (STAGE == 1) k_weights<Q, D, P><<<dim3(nnear3, Q), 256, 0, s>>>(A, d_near3, nnear3, half);
+        else k_gather<Q, D, P><<<dim3(nnear3, Q), 256, 0, s>>>(A, d_near3, nnear3, half);
+        DBM_LAUNCH_CHECK();
+      }
+      if (STAGE == 2 && fuse) {
+        if (nbricks3 > 0) {
+          const unsigned ge = (unsigned)std::min<int64_t>((int64_t)nbricks3 * 2, sm_count() * 4);
+          k_emit_bricks<Q><<<ge, 256, 0, s>>>(A, d_bricks3, half, nbricks3, d_fb3 + 4, d_fb3 + STAGE);
+          DBM_LAUNCH_CHECK();
+        }
+        if (nnear3 > 0) {
+          k_emit_bricks<Q><<<nnear3, 256, 0, s>>>(A, d_near3, half, nnear3, nullptr, nullptr);
+          DBM_LAUNCH_CHECK();
+        }
+      }
+    }
     return DBM_OK;
   }
 
@@ -1931,8 +2042,10 @@ struct SimImpl : SimBase {
       return DBM_ERR_STATE;
     }
     A.want_wexp = untiled ? 1 : 0;
-    A.odd_f = d_fb ? d_fb + 3 : nullptr;
-    if (d_fb) DBM_CUDA(cudaMemsetAsync(d_fb, 0, 4 * sizeof(int), s));  // fallback counts of the three stages, odd_f
+    // fallback counts of the three stages, odd_f
+    int* const fb = brick3_path() ? d_fb3 : d_fb;
+    A.odd_f = fb ? fb + 3 : nullptr;
+    if (fb) DBM_CUDA(cudaMemsetAsync(fb, 0, 4 * sizeof(int), s));
     k_collide<Q, D, P><<<gm, 256, 0, s>>>(A);
     DBM_LAUNCH_CHECK();
     if (untiled) {
@@ -1972,6 +2085,8 @@ struct SimImpl : SimBase {
       } else {
         k_thin_refine<Q, D, P><<<nbricks, 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
       }
+    } else if (brick3_path()) {
+      DBM_TRY(launch_brick3<0>(A, 0, s));
     } else {
       k_thin_refine<Q, D, P><<<nbricks, 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
     }
@@ -2043,6 +2158,8 @@ struct SimImpl : SimBase {
       } else {
         k_weights<Q, D, P><<<dim3(nbricks, Q), 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
       }
+    } else if (brick3_path()) {
+      DBM_TRY(launch_brick3<1>(A, 0, s));
     } else {
       k_weights<Q, D, P><<<dim3(nbricks, Q), 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
     }
@@ -2053,7 +2170,7 @@ struct SimImpl : SimBase {
     // intermediates, emits the points without an empty direction itself
     bool dense = false;
     if constexpr (D == 2 && std::is_same<P, PF32>::value) dense = (tiled_path() && shift_ok && use_shift && use_dense) || grid_path();
-    const int fuse = dense && !A.write_trace ? 1 : 0;
+    const int fuse = (dense || brick3_path()) && !A.write_trace ? 1 : 0;
     if (!dense) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (D == 2) {
       if (tiled_path()) {
@@ -2085,6 +2202,8 @@ struct SimImpl : SimBase {
       } else {
         k_gather<Q, D, P><<<dim3(nbricks, Q), 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
       }
+    } else if (brick3_path()) {
+      DBM_TRY(launch_brick3<2>(A, fuse, s));
     } else {
       k_gather<Q, D, P><<<dim3(nbricks, Q), 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
     }
@@ -2099,6 +2218,7 @@ struct SimImpl : SimBase {
 
   int step(int n, cudaStream_t s) override {
     if (n <= 0) return DBM_OK;
+    DBM_TRY(make_bricks3());
     ++version;
     DBM_CUDA(cudaEventRecord(ev_in, s));
     DBM_CUDA(cudaStreamWaitEvent(own, ev_in, 0));
@@ -2134,6 +2254,7 @@ struct SimImpl : SimBase {
   // receives the 6 stage durations (collide, thin+refine, compaction+sort+finalize, weights,
   // gather, emit) measured on the stream the kernels run on.
   int profile_step(float* stage_ms, cudaStream_t s) override {
+    DBM_TRY(make_bricks3());
     ++version;
     cudaEvent_t ev[7];
     for (auto& e : ev) DBM_CUDA(cudaEventCreate(&e));
@@ -2155,6 +2276,7 @@ struct SimImpl : SimBase {
   }
 
   int step_partial(int upto, cudaStream_t s) override {
+    DBM_TRY(make_bricks3());
     trace_on = 1;
     ++version;
     DBM_CUDA(cudaEventRecord(ev_in, s));
@@ -2171,6 +2293,7 @@ struct SimImpl : SimBase {
   // One full step launched stage by stage with every intermediate kept, and `h` called before the
   // collision and after the emit (the adjoint records its tape there).
   int step_hooked(StepHook* h, cudaStream_t s) override {
+    DBM_TRY(make_bricks3());
     const int keep = trace_on;
     ++version;
     trace_on = 1;
@@ -2271,6 +2394,7 @@ struct SimImpl : SimBase {
   int push_instances() {
     DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the table
     DBM_CUDA(cudaMemcpy(dinst, inst_h.data(), sizeof(InstK) * inst_h.size(), cudaMemcpyHostToDevice));
+    bricks3_stale = true;
     int any = 0;
     for (auto& I : inst_h) any |= I.has_obs;
     if (any != args.any_obstacle) {
