@@ -65,8 +65,14 @@ __device__ __forceinline__ void lbm_block_rows(int nj, int* r, int* j0, int* j1)
   *j1 = min(*j0 + kLbmRows, nj);
 }
 
-// FP64: BGK with the reference's formula (direbm/lbm.py:44-62: rho = sum f, u = sum f c / rho,
-// f += (feq - f) / tau), the divisions by rho and tau taken as products with one reciprocal each.
+// FP64: BGK (direbm/lbm.py:44-62: rho = sum f, u = sum f c / rho, f += (feq - f) / tau) with D2Q7's
+// structure written out, because GB300 runs FP64 at two lanes per clock and SM and the kernel is bound by
+// its FP64 operations.  The axes c = (1, 0), (1/2, s), (-1/2, s) and their opposites share their even part,
+//   feq_k - f_k = (rho W - f_k) + rho W (8 (c_k u)^2 - 2 u^2 +- 4 c_k u):
+// about 61 operations per node against 124 of the generic sums with their products by zero and one, and
+// fewer roundings of the size of feq (rms error against exact arithmetic at tau 0.55 / 0.7 / 1, times 1e-17:
+// 5.8 / 4.6 / 3.1 -> 3.6 / 2.9 / 2.2).
+// 1.57 M nodes: 331 -> 211 us a step; 61 operations at that rate take 164 us, the bytes 26 us.
 template <class IDX>
 __global__ void __launch_bounds__(256) k_lbm_f64(const double* __restrict__ src, double* __restrict__ dst, int ni,
                                                  int nj, const double* __restrict__ taus, LatK<7, 2> L) {
@@ -74,29 +80,34 @@ __global__ void __launch_bounds__(256) k_lbm_f64(const double* __restrict__ src,
   int r, j0, j1;
   lbm_block_rows(nj, &r, &j0, &j1);
   if (i >= ni) return;
-  const double inv_tau = 1.0 / taus[r];  // uniform in the block: one divide per thread row group
+  const double omega = 1.0 / taus[r];  // uniform in the block: once per thread
+  const double s = L.c[2][1], w0 = L.w[0], w = L.w[1];
   const IDX plane = (IDX)ni * nj;
-  const double* s = src + (IDX)r * 7 * plane;
+  const double* sp = src + (IDX)r * 7 * plane;
   double* d = dst + (IDX)r * 7 * plane;
   for (int j = j0; j < j1; ++j) {
     const HexNbr<IDX> nb(i, j, ni, nj);
     double f[7];
 #pragma unroll
-    for (int k = 0; k < 7; ++k) f[k] = s[(IDX)k * plane + nb.row[1] + i];
-    double rho = 0, mx = 0, my = 0;
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      rho += f[k];
-      mx += f[k] * L.c[k][0];
-      my += f[k] * L.c[k][1];
-    }
+    for (int k = 0; k < 7; ++k) f[k] = sp[(IDX)k * plane + nb.row[1] + i];
+    // axes 1-4, 2-5, 3-6: differences and sums
+    const double d1 = f[1] - f[4], d2 = f[2] - f[5], d3 = f[3] - f[6];
+    const double rho = f[0] + ((f[1] + f[4]) + ((f[2] + f[5]) + (f[3] + f[6])));
     const double ir = 1.0 / rho;
-    const double u[2] = {mx * ir, my * ir};
-    double feq[7];
-    equilibrium_all<7, 2, double>(rho, u, L, feq);
+    const double ux = fma(0.5, d2 - d3, d1) * ir, uy = (s * (d2 + d3)) * ir;
+    const double hx = 0.5 * ux, sy = s * uy;
+    const double cu[3] = {ux, hx + sy, sy - hx};
+    const double u2 = -2.0 * fma(uy, uy, ux * ux);
+    const double a = rho * w, a0 = rho * w0;
     double out[7];
+    out[0] = fma(omega, fma(a0, u2, a0 - f[0]), f[0]);
 #pragma unroll
-    for (int k = 0; k < 7; ++k) out[k] = f[k] + (feq[k] - f[k]) * inv_tau;
+    for (int q = 0; q < 3; ++q) {
+      const double even = fma(8.0, cu[q] * cu[q], u2);
+      const double up = fma(4.0, cu[q], even), down = fma(-4.0, cu[q], even);
+      out[q + 1] = fma(omega, fma(a, up, a - f[q + 1]), f[q + 1]);
+      out[q + 4] = fma(omega, fma(a, down, a - f[q + 4]), f[q + 4]);
+    }
     HexStore<IDX, 0>::put(d, plane, nb, out);
   }
 }
