@@ -23,7 +23,7 @@
 #include <limits>
 #include <vector>
 
-#include "sim.cuh"
+#include "sim_f64.cuh"
 #include "sortscan.cuh"
 
 namespace dbm {
@@ -133,8 +133,10 @@ template <class P>
 constexpr int thin_min_blocks() { return std::is_same<P, PF64>::value ? 1 : 6; }
 
 // Thinning + refine of one cell F of instance I (the untiled window kernels).
+// T: the block's shift table (FP64).
 template <int Q, int D, class P>
-__device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const uint32_t F, const InstK& I) {
+__device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const uint32_t F, const InstK& I,
+                                                 const ShiftTable<Q, D>* T = nullptr) {
   using real = typename P::real;
   int Fc[3];
   decode_cell<D>(I, F, Fc);
@@ -160,6 +162,18 @@ __device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const u
           const uint32_t m0 = A.a.start[Sg], m1 = A.a.start[Sg + 1];
           for (uint32_t m = m0; m < m1; ++m) {
             if (A.any_obstacle && ((A.bmask[m] >> k) & 1u)) continue;  // bounced: stays in its cell
+            if constexpr (std::is_same<P, PF64>::value) {  // far from landing here: no FP64 work
+              const float4 q = A.a.pf[m];
+              const float tf[3] = {q.x, q.y, q.z};
+              bool near = true;
+#pragma unroll
+              for (int a = 0; a < D; ++a) {
+                const float x = tf[a] + A.L.cdf[k][a] + (float)so[a];
+                const float t = 1e-3f + 1e-6f * fabsf(A.L.cdf[k][a]);
+                near &= x > -t && x < 1.f + t;
+              }
+              if (!near) continue;
+            }
             const PackItem<real> it = A.a.pk[m];  // the offsets in one load
             const real om[3] = {it.x, it.y, it.z};
             real t[3];
@@ -197,6 +211,7 @@ __device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const u
   }
   if (cnt == 0) {
     A.occ[F] = 0u;
+    A.fkey[F] = 0xffffffffu;  // read by the placement's neighbourhood search
     if (A.kappa_soft > 0) A.occ[A.ncells + F] = 0u;
     if (A.write_trace) { A.tcnt[F] = 0u; A.mask[F] = 0u; }
     return;
@@ -216,6 +231,55 @@ __device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const u
   float swf = 0.f, sxf[3] = {0.f, 0.f, 0.f};
   // soft spawn: sum of the components' direction vectors, FP64 (regular ones as count * c_k)
   double csr[3] = {0, 0, 0}, csb[3] = {0, 0, 0};
+  if constexpr (std::is_same<P, PF64>::value) {
+    // Listed over several directions in order and worked off together by the warp's lanes: a list worked
+    // off by a lane on its own would hold up the others.
+    const unsigned lanes = __activemask();
+    NearList list;
+    int nk = 0, kn = 0;  // hits of direction kn so far
+    auto done = [&](int k) {
+      if (A.kappa_soft > 0 && nk > 0) {
+#pragma unroll
+        for (int a = 0; a < D; ++a) csr[a] = __dadd_rn(csr[a], __dmul_rn((double)nk, A.L.c[kn][a]));
+      }
+      nk = 0;
+      kn = k;
+    };
+    auto flush = [&] {
+#pragma unroll 1
+      for (int i = 0; i < list.n; ++i) {
+        const int m = list.m[i];
+        const short4 s = list.s[i];
+        double e[3];
+        if (!le_bits(listed_d2<Q, D>(A.L, *T, A.a.pk[m], s, cen, e), A.R2)) continue;
+        if (s.w != kn) done(s.w);
+        mask |= 1u << s.w;
+        ++nk;
+        const double w = A.wexp[(int64_t)s.w * A.mcap + m];
+        // separate rounding of product and sum (no FMA), in loop order: the oracle reproduces this
+        // sum bit for bit
+        swd = __dadd_rn(swd, w);
+#pragma unroll
+        for (int a = 0; a < D; ++a) sxd[a] = __dadd_rn(sxd[a], __dmul_rn(w, e[a]));
+      }
+      list.n = 0;
+    };
+#pragma unroll 1
+    for (int k = 0; k < Q; ++k) {
+      float r[3] = {0.f, 0.f, 0.f};
+      int ctr[3] = {0, 0, 0};
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        r[a] = (float)cen[a] - A.L.cdf[k][a];
+        ctr[a] = -cd_cells(A.L, k, a);
+      }
+      near_items<D>(I, Fc, r, (float)A.R, k, ctr, A.a.start, A.a.pf, list,
+                    [&](uint32_t m) { return A.any_obstacle && ((A.bmask[m] >> k) & 1u); }, flush);
+      if (__any_sync(lanes, list.n > kNearFlush)) flush();
+    }
+    flush();
+    done(0);
+  } else {
 #pragma unroll 1
   for (int k = 0; k < Q; ++k) {
     int nk = 0;
@@ -274,17 +338,9 @@ __device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const u
               mask |= 1u << k;
               ++nk;
               const real w = A.want_wexp ? A.wexp[(int64_t)k * A.mcap + m] : exp(fstar_at<Q, D, P>(A, m, k));
-              if constexpr (std::is_same<P, PF64>::value) {
-                // separate rounding of product and sum (no FMA), in loop order: the oracle
-                // reproduces this sum bit for bit
-                swd = __dadd_rn(swd, w);
+              swf += w;
 #pragma unroll
-                for (int a = 0; a < D; ++a) sxd[a] = __dadd_rn(sxd[a], __dmul_rn(w, e[a]));
-              } else {
-                swf += w;
-#pragma unroll
-                for (int a = 0; a < D; ++a) sxf[a] = fmaf(w, e[a], sxf[a]);
-              }
+              for (int a = 0; a < D; ++a) sxf[a] = fmaf(w, e[a], sxf[a]);
             }
           }
         });
@@ -293,6 +349,7 @@ __device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const u
 #pragma unroll
       for (int a = 0; a < D; ++a) csr[a] = __dadd_rn(csr[a], __dmul_rn((double)nk, A.L.c[k][a]));
     }
+  }
   }
   if (A.any_obstacle && I.has_obs && sphere_dist2<D, real>(I, Fc, cen) < I.reach2) {
     // bounced components (displacement 0, opposite label): window order, then moment, then slot
@@ -448,15 +505,29 @@ __device__ __forceinline__ void thin_refine_cell(const Args<Q, D, P>& A, const u
 // The untiled window kernels take one brick of cells per block (thread t <-> cell t of the brick):
 // a block's windows then cover a compact region that stays in L1, where consecutive points in cell
 // order would span a long strip of rows.
+// FP64: a block takes a quarter of a brick (64 threads), so that a small box fills the GPU.
 template <int Q, int D, class P>
 __global__ void __launch_bounds__(256, thin_min_blocks<P>()) k_thin_refine(const __grid_constant__ Args<Q, D, P> A,
                                                                            const Brick* __restrict__ bricks,
                                                                            int nbricks, BrickGeo bg) {
-  for (int bi = blockIdx.x; bi < nbricks; bi += gridDim.x) {
-    const Brick B = bricks[bi];
-    const InstK I = A.inst[B.inst];
-    uint32_t F;
-    if (brick_cell<D>(B, I, bg, threadIdx.x, &F)) thin_refine_cell<Q, D, P>(A, F, I);
+  if constexpr (std::is_same<P, PF64>::value) {
+    __shared__ ShiftTable<Q, D> T;
+    T.fill(A.L);
+    __syncthreads();
+    const int parts = 256 / blockDim.x;
+    for (int u = blockIdx.x; u < nbricks * parts; u += gridDim.x) {
+      const Brick B = bricks[u / parts];
+      const InstK I = A.inst[B.inst];
+      uint32_t F;
+      if (brick_cell<D>(B, I, bg, (u % parts) * blockDim.x + threadIdx.x, &F)) thin_refine_cell<Q, D, P>(A, F, I, &T);
+    }
+  } else {
+    for (int bi = blockIdx.x; bi < nbricks; bi += gridDim.x) {
+      const Brick B = bricks[bi];
+      const InstK I = A.inst[B.inst];
+      uint32_t F;
+      if (brick_cell<D>(B, I, bg, threadIdx.x, &F)) thin_refine_cell<Q, D, P>(A, F, I);
+    }
   }
 }
 
@@ -475,6 +546,7 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ Args<Q, D,
     it.z = D > 2 ? S.off[2 * stride + i] : (real)0;
     it.cx = (real)((g - I.base) % (uint32_t)I.dims[0]);
     S.pk[i] = it;
+    if constexpr (std::is_same<P, PF64>::value) S.pf[i] = make_float4((float)it.x, (float)it.y, (float)it.z, __int_as_float((int)it.cx));
   }
 }
 
@@ -592,10 +664,45 @@ static void launch_cell_start(const uint32_t* keys, const uint32_t* d_n, uint32_
 // sw of component (m, k), m a moment in cell g of instance I.
 template <int Q, int D, class P>
 __device__ __forceinline__ void weights_one(const Args<Q, D, P>& A, const uint32_t m, const int k, const uint32_t g,
-                                            const InstK& I) {
+                                            const InstK& I, const ShiftTable<Q, D>* T = nullptr) {
   using real = typename P::real;
   int Sc[3];
   decode_cell<D>(I, g, Sc);
+  if constexpr (std::is_same<P, PF64>::value) {
+    const bool stays = A.any_obstacle && ((A.bmask[m] >> k) & 1u);  // bounced: at the moment
+    double o[3] = {0, 0, 0};
+    float r[3] = {0.f, 0.f, 0.f};
+    int ctr[3] = {0, 0, 0};
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      o[a] = A.a.off[(int64_t)a * A.mcap + m];
+      r[a] = (float)o[a] + (stays ? 0.f : A.L.cdf[k][a]);
+      ctr[a] = stays ? 0 : cd_cells(A.L, k, a);
+    }
+    double swd = 0;
+    NearList list;
+    auto flush = [&] {
+#pragma unroll 1
+      for (int i = 0; i < list.n; ++i) {
+        const PackItem<double> it = A.b.pk[list.m[i]];
+        const short4 s = list.s[i];
+        const int j[3] = {-s.x, -s.y, -s.z};
+        const double off[3] = {it.x, it.y, it.z};
+        double cc[3] = {0, 0, 0}, e[3];
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+          cc[a] = rn_sub(stays ? (double)j[a] : T->at(A.L, k, a, j[a]), off[a]);
+        const double d2 = canon_d2<D, double>(o, cc, e);
+        if (le_bits(d2, A.R2)) swd += A.R - rn_sqrt(d2);
+      }
+      list.n = 0;
+    };
+    const unsigned lanes = __activemask();
+    near_items<D>(I, Sc, r, (float)A.R, k, ctr, A.b.start, A.b.pf, list, [](uint32_t) { return false; }, flush);
+    __syncwarp(lanes);
+    flush();
+    A.sw[(int64_t)k * A.mcap + m] = swd > 0 ? 1 / swd : 0;  // stored inverted
+  } else {
   real o[3] = {0, 0, 0}, cdk[3] = {0, 0, 0};
   int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   const bool bounced = A.any_obstacle && ((A.bmask[m] >> k) & 1u);  // stays at the moment
@@ -607,7 +714,6 @@ __device__ __forceinline__ void weights_one(const Args<Q, D, P>& A, const uint32
     lo[a] = (int)floor(t - A.R - A.tiny);
     hi[a] = (int)floor(t + A.R + A.tiny);
   }
-  double swd = 0;
   CSum sws;
   // window rows (gz, gy) in order; per row one x range narrowed by the row's smallest |e_y|, |e_z|,
   // visited as runs of consecutive cells (the items of a run are contiguous, in cell order); the
@@ -656,19 +762,17 @@ __device__ __forceinline__ void weights_one(const Args<Q, D, P>& A, const uint32
           real e[3];
           const real d2 = canon_d2<D, real>(o, cc, e);
           if (d2 <= A.R2) {
-            const real d = rn_sqrt(d2);
-            if constexpr (std::is_same<P, PF64>::value) swd += A.R - d; else sws.add(A.R - d);
+            sws.add(A.R - rn_sqrt(d2));
           }
         }
       });
     }
-  real sw;
-  if constexpr (std::is_same<P, PF64>::value) sw = swd; else sw = sws.value();
+  const real sw = sws.value();
   const real inv = sw > (real)0 ? (real)1 / sw : (real)0;  // stored inverted
   const int64_t i = (int64_t)k * A.mcap + m;
   A.sw[i] = inv;
-  if constexpr (std::is_same<P, PF64>::value) A.kv[i] = KV<real>{inv, A.a.f64[i]};
-  else A.kv[i] = KV<real>{inv, A.a.dev[i]};
+  A.kv[i] = KV<real>{inv, A.a.dev[i]};
+  }
 }
 
 // FP32: six resident blocks per SM (the gather waits on loads and needs the warps); FP64 keeps its
@@ -679,7 +783,7 @@ constexpr int gather_min_blocks() { return std::is_same<P, PF64>::value ? 1 : 6;
 // Resampled f_k of control point j, in cell G of instance I.
 template <int Q, int D, class P>
 __device__ __forceinline__ void gather_one(const Args<Q, D, P>& A, const uint32_t j, const int k, const uint32_t G,
-                                           const InstK& I) {
+                                           const InstK& I, const ShiftTable<Q, D>* T = nullptr) {
   using real = typename P::real;
   int Gc[3];
   decode_cell<D>(I, G, Gc);
@@ -696,6 +800,33 @@ __device__ __forceinline__ void gather_one(const Args<Q, D, P>& A, const uint32_
   double acc = 0;
   CSum sa;
   float sb = 0.f;  // deviation part: small, plain FMA accumulation suffices
+  if constexpr (std::is_same<P, PF64>::value) {
+    float r[3] = {0.f, 0.f, 0.f};
+    int ctr[3] = {0, 0, 0};
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      r[a] = (float)p[a] - A.L.cdf[k][a];
+      ctr[a] = -cd_cells(A.L, k, a);
+    }
+    const unsigned lanes = __activemask();
+    NearList list;
+    auto flush = [&] {
+#pragma unroll 1
+      for (int i = 0; i < list.n; ++i) {
+        const int64_t m = list.m[i];
+        double e[3];
+        const double d2 = listed_d2<Q, D>(A.L, *T, A.a.pk[m], list.s[i], p, e);
+        if (!le_bits(d2, A.R2)) continue;
+        const double inv = A.sw[(int64_t)k * A.mcap + m];
+        if (__double_as_longlong(inv) > 0) acc += ((A.R - rn_sqrt(d2)) * inv) * A.a.f64[(int64_t)k * A.mcap + m];
+      }
+      list.n = 0;
+    };
+    near_items<D>(I, Gc, r, (float)A.R, k, ctr, A.a.start, A.a.pf, list,
+                  [&](uint32_t m) { return A.any_obstacle && ((A.bmask[m] >> k) & 1u); }, flush);
+    __syncwarp(lanes);
+    flush();
+  } else {
   const real bxr = p[0] - cdk[0];
   // window rows (sz, sy) in order; per row one x range narrowed by the row's smallest |e_y|, |e_z|,
   // visited as runs of consecutive cells (the items of a run are contiguous, in cell order); the
@@ -744,17 +875,14 @@ __device__ __forceinline__ void gather_one(const Args<Q, D, P>& A, const uint32_
             const KV<real> kv = A.kv[(int64_t)k * A.mcap + m];
             if (kv.inv > (real)0) {
               const real wgt = (A.R - rn_sqrt(d2)) * kv.inv;
-              if constexpr (std::is_same<P, PF64>::value) {
-                acc += wgt * kv.f;
-              } else {
-                sa.add_prod(wgt, A.a.rho[m]);
-                sb = __fmaf_rn(wgt, kv.f, sb);
-              }
+              sa.add_prod(wgt, A.a.rho[m]);
+              sb = __fmaf_rn(wgt, kv.f, sb);
             }
           }
         }
       });
     }
+  }
   if (A.any_obstacle && k > 0 && I.has_obs && sphere_dist2<D, real>(I, Gc, p) < I.reach2) {
     // components of slot kb = opp[k] that bounced carry label k and sit at their moment's offset
     const int kb = A.L.opp[k];
@@ -784,14 +912,15 @@ __device__ __forceinline__ void gather_one(const Args<Q, D, P>& A, const uint32_
             for (int a = 0; a < D; ++a) o[a] = A.a.off[(int64_t)a * A.mcap + m];
             const real d2 = canon_d2<D, real>(o, c, e);
             if (d2 > A.R2) continue;
-            const KV<real> kv = A.kv[(int64_t)kb * A.mcap + m];
-            if (kv.inv > (real)0) {
-              const real wgt = (A.R - rn_sqrt(d2)) * kv.inv;
+            const int64_t ib = (int64_t)kb * A.mcap + m;
+            const real inv = A.sw[ib];
+            if (inv > (real)0) {
+              const real wgt = (A.R - rn_sqrt(d2)) * inv;
               if constexpr (std::is_same<P, PF64>::value) {
-                acc += wgt * kv.f;
+                acc += wgt * A.a.f64[ib];
               } else {
                 sa.add_prod(wgt, A.a.rho[m]);
-                sb = __fmaf_rn(wgt, kv.f, sb);
+                sb = __fmaf_rn(wgt, A.a.dev[ib], sb);
               }
             }
           }
@@ -813,17 +942,31 @@ __device__ __forceinline__ void gather_one(const Args<Q, D, P>& A, const uint32_
   if (empty) atomicOr(A.emask + j, 1u << k);
 }
 
+// FP64: the block's shift table, filled (every thread calls); nothing otherwise.
+template <int Q, int D, class P>
+__device__ __forceinline__ const ShiftTable<Q, D>* block_shifts(const LatK<Q, D>& L) {
+  if constexpr (std::is_same<P, PF64>::value) {
+    __shared__ ShiftTable<Q, D> T;
+    T.fill(L);
+    __syncthreads();
+    return &T;
+  } else {
+    return nullptr;
+  }
+}
+
 template <int Q, int D, class P>
 __global__ void __launch_bounds__(256, gather_min_blocks<P>()) k_weights(const __grid_constant__ Args<Q, D, P> A,
                                                                          const Brick* __restrict__ bricks, int nbricks,
                                                                          BrickGeo bg) {
   const int k = blockIdx.y;
+  const ShiftTable<Q, D>* T = block_shifts<Q, D, P>(A.L);
   for (int bi = blockIdx.x; bi < nbricks; bi += gridDim.x) {
     const Brick B = bricks[bi];
     const InstK I = A.inst[B.inst];
     uint32_t F;
     if (!brick_cell<D>(B, I, bg, threadIdx.x, &F)) continue;
-    for (uint32_t m = A.a.start[F], m1 = A.a.start[F + 1]; m < m1; ++m) weights_one<Q, D, P>(A, m, k, F, I);
+    for (uint32_t m = A.a.start[F], m1 = A.a.start[F + 1]; m < m1; ++m) weights_one<Q, D, P>(A, m, k, F, I, T);
   }
 }
 
@@ -832,12 +975,13 @@ __global__ void __launch_bounds__(256, gather_min_blocks<P>()) k_gather(const __
                                                                         const Brick* __restrict__ bricks, int nbricks,
                                                                         BrickGeo bg) {
   const int k = blockIdx.y;
+  const ShiftTable<Q, D>* T = block_shifts<Q, D, P>(A.L);
   for (int bi = blockIdx.x; bi < nbricks; bi += gridDim.x) {
     const Brick B = bricks[bi];
     const InstK I = A.inst[B.inst];
     uint32_t F;
     if (!brick_cell<D>(B, I, bg, threadIdx.x, &F)) continue;
-    for (uint32_t j = A.b.start[F], j1 = A.b.start[F + 1]; j < j1; ++j) gather_one<Q, D, P>(A, j, k, F, I);
+    for (uint32_t j = A.b.start[F], j1 = A.b.start[F + 1]; j < j1; ++j) gather_one<Q, D, P>(A, j, k, F, I, T);
   }
 }
 
@@ -1426,6 +1570,7 @@ struct SimImpl : SimBase {
       DBM_TRY(alloc(&S.off, (int64_t)D * cap));
       DBM_TRY(alloc(&S.pk, cap));
       if constexpr (std::is_same<P, PF64>::value) {
+        DBM_TRY(alloc(&S.pf, cap));
         DBM_TRY(alloc(&S.f64, (int64_t)Q * cap));
       } else {
         DBM_TRY(alloc(&S.rho, cap));
@@ -1486,6 +1631,7 @@ struct SimImpl : SimBase {
     DBM_TRY(alloc(&A.sw, (int64_t)Q * mcap));
     A.kv = nullptr;  // the untiled path's buffers: see ensure_untiled
     A.wexp = nullptr;
+    if constexpr (std::is_same<P, PF64>::value) A.wexp = A.sw;  // read by the refine before the weights take sw
     A.want_wexp = 0;
     if constexpr (std::is_same<P, PF64>::value) {
       DBM_TRY(alloc(&A.cpf64, (int64_t)Q * ccap));
@@ -1656,6 +1802,7 @@ struct SimImpl : SimBase {
   // ([Q][mcap] each).  Allocated by the calls that make that path possible (creation in 3D, an
   // obstacle, the soft spawn, tiles off), so a tiled 2D simulation never holds them.
   int ensure_untiled() override {
+    if constexpr (std::is_same<P, PF64>::value) return DBM_OK;  // reads 1/sw and f* where they are
     if (args.kv) return DBM_OK;
     DBM_TRY(alloc(&args.kv, (int64_t)Q * mcap));
     DBM_TRY(alloc(&args.wexp, (int64_t)Q * mcap));
@@ -1732,7 +1879,7 @@ struct SimImpl : SimBase {
     geo.cp = c;
     const int mcells = (geo.tx + m.xh - m.xl) * (geo.ty + m.yh - m.yl);
     const int ccells = (geo.tx + c.xh - c.xl) * (geo.ty + c.yh - c.yl);
-    const size_t budget = std::is_same<P, PF64>::value ? 112 * 1024 : 56 * 1024;
+    const size_t budget = 56 * 1024;
     geo.cap_tile = 2 * geo.tx * geo.ty;
     geo.cap_refine = pick_cap(0, mcells, budget);
     geo.cap_weights = pick_cap(1, ccells, budget);
@@ -1792,7 +1939,7 @@ struct SimImpl : SimBase {
       DBM_TRY(alloc(&d_fb, (int64_t)ntiles + 4));
       DBM_CUDA(cudaMemset(d_fb, 0, ((size_t)ntiles + 4) * sizeof(int)));
     }
-    if constexpr (D == 2) {
+    if constexpr (kTiles) {
       DBM_CUDA(cudaFuncSetAttribute((const void*)k_thin_refine_t<Q, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sm_refine));
       DBM_CUDA(cudaFuncSetAttribute((const void*)k_weights_t<Q, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1804,60 +1951,58 @@ struct SimImpl : SimBase {
       DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], k_weights_t<Q, P>, 256, sm_weights));
       DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[2], k_gather_t<Q, P>, 256, sm_gather));
       for (int i = 0; i < 3; ++i) pgrid[i] = std::max(1, std::min(ntiles, std::max(nb[i], 1) * sm_count()));
-      if constexpr (std::is_same<P, PF32>::value) {
-        if (grid_w) {
-          const void* kg[3];
-          with_grid([&](auto w) {
-            kg[0] = (const void*)k_thin_refine_grid<Q, w.value>;
-            kg[1] = (const void*)k_weights_grid<Q, w.value>;
-            kg[2] = (const void*)k_gather_grid<Q, w.value>;
-          });
-          const void* kf[3] = {(const void*)k_grid_fallback<Q, 0>, (const void*)k_grid_fallback<Q, 1>,
-                               (const void*)k_grid_fallback<Q, 2>};
-          const size_t sf[3] = {sm_refine, sm_weights, sm_gather};
-          for (int i = 0; i < 3; ++i) {
-            DBM_CUDA(cudaFuncSetAttribute(kg[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_grid[i]));
-            DBM_CUDA(cudaFuncSetAttribute(kf[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf[i]));
-            int nbd = 1;
-            DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kg[i], 256, sm_grid[i]));
-            pgrid_grid[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
-          }
+      if (grid_w) {
+        const void* kg[3];
+        with_grid([&](auto w) {
+          kg[0] = (const void*)k_thin_refine_grid<Q, w.value>;
+          kg[1] = (const void*)k_weights_grid<Q, w.value>;
+          kg[2] = (const void*)k_gather_grid<Q, w.value>;
+        });
+        const void* kf[3] = {(const void*)k_grid_fallback<Q, 0>, (const void*)k_grid_fallback<Q, 1>,
+                             (const void*)k_grid_fallback<Q, 2>};
+        const size_t sf[3] = {sm_refine, sm_weights, sm_gather};
+        for (int i = 0; i < 3; ++i) {
+          DBM_CUDA(cudaFuncSetAttribute(kg[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_grid[i]));
+          DBM_CUDA(cudaFuncSetAttribute(kf[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf[i]));
+          int nbd = 1;
+          DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kg[i], 256, sm_grid[i]));
+          pgrid_grid[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
         }
-        if (shift_ok) {
-          DBM_CUDA(cudaFuncSetAttribute((const void*)k_gather_ts<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sm_gather_s));
-          int nbs = 1;
-          DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbs, k_gather_ts<Q>, 256, sm_gather_s));
-          pgrid_s = std::max(1, std::min(ntiles, std::max(nbs, 1) * sm_count()));
-          DBM_CUDA(cudaFuncSetAttribute((const void*)k_thin_refine_t<Q, P, true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
-          int nbr = 1;
-          DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbr, k_thin_refine_t<Q, P, true>, 256, sm_refine));
-          pgrid_rs = std::max(1, std::min(ntiles, std::max(nbr, 1) * sm_count()));
-          DBM_CUDA(cudaFuncSetAttribute((const void*)k_weights_t<Q, P, true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_weights));
-          int nbw = 1;
-          DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbw, k_weights_t<Q, P, true>, 256, sm_weights));
-          pgrid_ws = std::max(1, std::min(ntiles, std::max(nbw, 1) * sm_count()));
-          const void* kds[3];
-          with_near([&](auto tx) {
-            kds[0] = (const void*)k_thin_refine_ds<Q, tx.value>;
-            kds[1] = (const void*)k_weights_ds<Q, tx.value>;
-            kds[2] = (const void*)k_gather_ds<Q, tx.value>;
-          });
-          for (int i = 0; i < 3; ++i) {
-            DBM_CUDA(cudaFuncSetAttribute(kds[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
-            int nbd = 1;
-            DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kds[i], 256, sm_ds[i]));
-            pgrid_ds[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
-          }
-          DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 0>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
-          DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 1>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_weights));
-          DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 2>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_gather_s));
+      }
+      if (shift_ok) {
+        DBM_CUDA(cudaFuncSetAttribute((const void*)k_gather_ts<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sm_gather_s));
+        int nbs = 1;
+        DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbs, k_gather_ts<Q>, 256, sm_gather_s));
+        pgrid_s = std::max(1, std::min(ntiles, std::max(nbs, 1) * sm_count()));
+        DBM_CUDA(cudaFuncSetAttribute((const void*)k_thin_refine_t<Q, P, true>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
+        int nbr = 1;
+        DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbr, k_thin_refine_t<Q, P, true>, 256, sm_refine));
+        pgrid_rs = std::max(1, std::min(ntiles, std::max(nbr, 1) * sm_count()));
+        DBM_CUDA(cudaFuncSetAttribute((const void*)k_weights_t<Q, P, true>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_weights));
+        int nbw = 1;
+        DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbw, k_weights_t<Q, P, true>, 256, sm_weights));
+        pgrid_ws = std::max(1, std::min(ntiles, std::max(nbw, 1) * sm_count()));
+        const void* kds[3];
+        with_near([&](auto tx) {
+          kds[0] = (const void*)k_thin_refine_ds<Q, tx.value>;
+          kds[1] = (const void*)k_weights_ds<Q, tx.value>;
+          kds[2] = (const void*)k_gather_ds<Q, tx.value>;
+        });
+        for (int i = 0; i < 3; ++i) {
+          DBM_CUDA(cudaFuncSetAttribute(kds[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
+          int nbd = 1;
+          DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kds[i], 256, sm_ds[i]));
+          pgrid_ds[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
         }
+        DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 0>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
+        DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 1>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_weights));
+        DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 2>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_gather_s));
       }
     }
     tiled = true;
@@ -2002,9 +2147,22 @@ struct SimImpl : SimBase {
     if (stage_ev) cudaEventRecord(stage_ev[i], s);
   }
 
-  // The tiled 2D kernels serve plain periodic/bounded boxes; obstacles and the soft spawn run on
-  // the untiled window kernels.
-  bool tiled_path() const { return D == 2 && tiled && use_tiles && !args.any_obstacle && args.kappa_soft == 0; }
+  // The tiled 2D kernels serve plain periodic/bounded boxes in FP32; obstacles and the soft spawn run on
+  // the untiled window kernels, and so does FP64, where staging a tile saves nothing: its time is that of
+  // the FP64 units (sim_f64.cuh; 128 x 128 cells, ten steps: tiled 13.4 ms, untiled 3.5).
+  static constexpr bool kTiles = D == 2 && std::is_same<P, PF32>::value;
+  bool tiled_path() const { return kTiles && tiled && use_tiles && !args.any_obstacle && args.kappa_soft == 0; }
+  // Control points placed without a sort (2D): plain boxes, a small neighbourhood.
+  bool place_path() const {
+    return D == 2 && tiled && use_tiles && !args.any_obstacle && args.kappa_soft == 0 && place_h > 0;
+  }
+
+  // The untiled thinning + refine: FP64 in blocks of 64 threads (one warp to two of each brick on an SM
+  // keep its narrow FP64 units busy, and a 128 x 128 box then has 256 blocks instead of 64).
+  void launch_thin_refine(Args<Q, D, P>& A, cudaStream_t s) {
+    const int threads = std::is_same<P, PF64>::value ? 64 : 256;
+    k_thin_refine<Q, D, P><<<nbricks * (256 / threads), threads, 0, s>>>(A, d_bricks, nbricks, bgeo);
+  }
 
   // fn(integral constant): the tile width for the NEAR dense kernels, 0 where they do not apply.
   template <class Fn>
@@ -2037,7 +2195,7 @@ struct SimImpl : SimBase {
     // the untiled window kernels (3D, obstacles, the soft spawn, or tiles off) read packed items
     // and the refine weights exp(f*) precomputed by the collision
     const bool untiled = !tiled_path();
-    if (untiled && !A.kv) {
+    if (std::is_same<P, PF32>::value && untiled && !A.kv) {
       set_last_error("internal: the untiled window kernels' buffers were not allocated");
       return DBM_ERR_STATE;
     }
@@ -2054,41 +2212,39 @@ struct SimImpl : SimBase {
     }
     mark(1, s);
     if (upto <= 1) return DBM_OK;
-    if constexpr (D == 2) {
+    if constexpr (kTiles) {
       if (tiled_path()) {
         bool shifted = false;
-        if constexpr (std::is_same<P, PF32>::value) {
-          if (shift_ok && use_shift && use_dense) {
-            const int grid = use_persistent ? pgrid_ds[0] : ntiles;
-            with_near([&](auto tx) {
-              k_thin_refine_ds<Q, tx.value><<<grid, 256, sm_ds[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
-            });
-            DBM_LAUNCH_CHECK();
-            k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
-            shifted = true;
-          } else if (grid_path()) {
-            const int grid = use_persistent ? pgrid_grid[0] : ntiles;
-            with_grid([&](auto w) {
-              k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
-            });
-            DBM_LAUNCH_CHECK();
-            k_grid_fallback<Q, 0><<<pgrid[0], 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
-            shifted = true;
-          } else if (shift_ok && use_shift) {
-            k_thin_refine_t<Q, P, true><<<use_persistent ? pgrid_rs : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo,
-                                                                                                  ntiles);
-            shifted = true;
-          }
+        if (shift_ok && use_shift && use_dense) {
+          const int grid = use_persistent ? pgrid_ds[0] : ntiles;
+          with_near([&](auto tx) {
+            k_thin_refine_ds<Q, tx.value><<<grid, 256, sm_ds[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
+          });
+          DBM_LAUNCH_CHECK();
+          k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
+          shifted = true;
+        } else if (grid_path()) {
+          const int grid = use_persistent ? pgrid_grid[0] : ntiles;
+          with_grid([&](auto w) {
+            k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
+          });
+          DBM_LAUNCH_CHECK();
+          k_grid_fallback<Q, 0><<<pgrid[0], 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
+          shifted = true;
+        } else if (shift_ok && use_shift) {
+          k_thin_refine_t<Q, P, true><<<use_persistent ? pgrid_rs : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo,
+                                                                                                ntiles);
+          shifted = true;
         }
         if (!shifted)
           k_thin_refine_t<Q, P><<<use_persistent ? pgrid[0] : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo, ntiles);
       } else {
-        k_thin_refine<Q, D, P><<<nbricks, 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
+        launch_thin_refine(A, s);
       }
     } else if (brick3_path()) {
       DBM_TRY(launch_brick3<0>(A, 0, s));
     } else {
-      k_thin_refine<Q, D, P><<<nbricks, 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
+      launch_thin_refine(A, s);
     }
     DBM_LAUNCH_CHECK();
     mark(2, s);
@@ -2096,7 +2252,7 @@ struct SimImpl : SimBase {
     // slots: regular CPs [0, ncells), spawned ones [ncells, 2 ncells); the stable sort keeps that
     // order among CPs of one cell
     const unsigned gc = std::min<unsigned>(div_up(ccap, 256), (unsigned)sm_count() * 16);
-    if (!untiled && place_h > 0 && A.kappa_soft == 0) {
+    if (place_path()) {
       // counts per final cell -> cell starts (and P) by one scan -> each point's slot
       const unsigned gf = std::min<unsigned>(div_up(ncells, 256), (unsigned)sm_count() * 16);
       DBM_CUDA(cudaMemsetAsync(A.b.start, 0, ((size_t)ncells + 1) * 4, s));
@@ -2105,6 +2261,10 @@ struct SimImpl : SimBase {
       DBM_TRY(scan_exclusive_u32(A.b.start, A.b.start, (int64_t)ncells + 1, nullptr, A.d_P, place_tmp, s));
       k_place<Q, D, P><<<gf, 256, 0, s>>>(A, place_h, k_in, v_in);
       DBM_LAUNCH_CHECK();
+      if (untiled) {
+        k_pack<Q, D, P><<<gc, 256, 0, s>>>(A, A.b, A.ccap, A.d_P);
+        DBM_LAUNCH_CHECK();
+      }
       sorted_in_alt = false;
       A.skeys = k_in;
       A.svals = v_in;
@@ -2127,31 +2287,29 @@ struct SimImpl : SimBase {
     }
     mark(3, s);
     if (upto <= 3) return DBM_OK;
-    if constexpr (D == 2) {
+    if constexpr (kTiles) {
       if (tiled_path()) {
         bool shifted = false;
-        if constexpr (std::is_same<P, PF32>::value) {
-          if (shift_ok && use_shift && use_dense) {
-            const int grid = use_persistent ? pgrid_ds[1] : ntiles;
-            with_near([&](auto tx) {
-              k_weights_ds<Q, tx.value><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
-            });
-            DBM_LAUNCH_CHECK();
-            k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
-            shifted = true;
-          } else if (grid_path()) {
-            const int grid = use_persistent ? pgrid_grid[1] : ntiles;
-            with_grid([&](auto w) {
-              k_weights_grid<Q, w.value><<<grid, 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
-            });
-            DBM_LAUNCH_CHECK();
-            k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
-            shifted = true;
-          } else if (shift_ok && use_shift) {
-            k_weights_t<Q, P, true><<<use_persistent ? pgrid_ws : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo,
-                                                                                               ntiles);
-            shifted = true;
-          }
+        if (shift_ok && use_shift && use_dense) {
+          const int grid = use_persistent ? pgrid_ds[1] : ntiles;
+          with_near([&](auto tx) {
+            k_weights_ds<Q, tx.value><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+          });
+          DBM_LAUNCH_CHECK();
+          k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
+          shifted = true;
+        } else if (grid_path()) {
+          const int grid = use_persistent ? pgrid_grid[1] : ntiles;
+          with_grid([&](auto w) {
+            k_weights_grid<Q, w.value><<<grid, 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+          });
+          DBM_LAUNCH_CHECK();
+          k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
+          shifted = true;
+        } else if (shift_ok && use_shift) {
+          k_weights_t<Q, P, true><<<use_persistent ? pgrid_ws : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo,
+                                                                                             ntiles);
+          shifted = true;
         }
         if (!shifted)
           k_weights_t<Q, P><<<use_persistent ? pgrid[1] : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo, ntiles);
@@ -2169,33 +2327,31 @@ struct SimImpl : SimBase {
     // the dense gather writes every control point's empty mask and, unless the step keeps its
     // intermediates, emits the points without an empty direction itself
     bool dense = false;
-    if constexpr (D == 2 && std::is_same<P, PF32>::value) dense = (tiled_path() && shift_ok && use_shift && use_dense) || grid_path();
+    if constexpr (kTiles) dense = (tiled_path() && shift_ok && use_shift && use_dense) || grid_path();
     const int fuse = (dense || brick3_path()) && !A.write_trace ? 1 : 0;
     if (!dense) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
-    if constexpr (D == 2) {
+    if constexpr (kTiles) {
       if (tiled_path()) {
         bool shifted = false;
-        if constexpr (std::is_same<P, PF32>::value) {
-          if (shift_ok && use_shift && use_dense) {
-            const int grid = use_persistent ? pgrid_ds[2] : ntiles;
-            with_near([&](auto tx) {
-              k_gather_ds<Q, tx.value><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + 4, d_fb + 2, fuse);
-            });
-            DBM_LAUNCH_CHECK();
-            k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2, fuse);
-            shifted = true;
-          } else if (grid_path()) {
-            const int grid = use_persistent ? pgrid_grid[2] : ntiles;
-            with_grid([&](auto w) {
-              k_gather_grid<Q, w.value><<<grid, 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 2, fuse);
-            });
-            DBM_LAUNCH_CHECK();
-            k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 2, fuse);
-            shifted = true;
-          } else if (shift_ok && use_shift) {
-            k_gather_ts<Q><<<use_persistent ? pgrid_s : ntiles, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, ntiles);
-            shifted = true;
-          }
+        if (shift_ok && use_shift && use_dense) {
+          const int grid = use_persistent ? pgrid_ds[2] : ntiles;
+          with_near([&](auto tx) {
+            k_gather_ds<Q, tx.value><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + 4, d_fb + 2, fuse);
+          });
+          DBM_LAUNCH_CHECK();
+          k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2, fuse);
+          shifted = true;
+        } else if (grid_path()) {
+          const int grid = use_persistent ? pgrid_grid[2] : ntiles;
+          with_grid([&](auto w) {
+            k_gather_grid<Q, w.value><<<grid, 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 2, fuse);
+          });
+          DBM_LAUNCH_CHECK();
+          k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 2, fuse);
+          shifted = true;
+        } else if (shift_ok && use_shift) {
+          k_gather_ts<Q><<<use_persistent ? pgrid_s : ntiles, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, ntiles);
+          shifted = true;
         }
         if (!shifted)
           k_gather_t<Q, P><<<use_persistent ? pgrid[2] : ntiles, 256, sm_gather, s>>>(A, d_tiles, geo, ntiles);

@@ -54,6 +54,7 @@ struct StateP {
   uint32_t* cell = nullptr;   // [cap]
   real* off = nullptr;        // [D][cap]
   PackItem<real>* pk = nullptr;  // [cap] packed copy for the untiled window kernels
+  float4* pf = nullptr;          // FP64: [cap] the same rounded to float, for the candidate search
   double* f64 = nullptr;      // FP64: [Q][cap]
   float* rho = nullptr;       // FP32DEV: [cap]
   float* dev = nullptr;       // FP32DEV: [Q][cap]

@@ -184,7 +184,6 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
                                                  const int* s_gi, const Pair<typename P::real>* s_pos,
                                                  typename P::real* s_w, int nstaged) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int lx = threadIdx.x % G.tx, ly = threadIdx.x / G.tx;
   const int Fx = T.x0 + lx, Fy = T.y0 + ly;
   const bool valid = ly < G.ty && Fx < I.dims[0] && Fy < I.dims[1];
@@ -201,8 +200,7 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
   uint32_t cnt = 0;
   real cen[3] = {0, 0, 0};
   if (valid) {
-    real sum[2] = {0, 0};
-    CSum csum[2];
+      CSum csum[2];
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
       const real cdx = A.L.template cd_as<real>(k, 0), cdy = A.L.template cd_as<real>(k, 1);
@@ -223,32 +221,21 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
             if (tx >= fx0 && tx < fx0 + (real)1 && ty >= fy0 && ty < fy0 + (real)1) {
               ++cnt;
               const real rx = rn_add((real)sox, tx), ry = rn_add((real)soy, ty);
-              if constexpr (F64) {
-                sum[0] += rx;
-                sum[1] += ry;
-              } else {
-                csum[0].add(rx);
-                csum[1].add(ry);
-              }
+              csum[0].add(rx);
+              csum[1].add(ry);
             }
           }
         }
     }
     if (cnt) {
-      if constexpr (F64) {
-        cen[0] = sum[0] / (real)cnt;
-        cen[1] = sum[1] / (real)cnt;
-      } else {
-        cen[0] = csum[0].value() / (real)cnt;
-        cen[1] = csum[1].value() / (real)cnt;
-      }
+      cen[0] = csum[0].value() / (real)cnt;
+      cen[1] = csum[1].value() / (real)cnt;
     }
   }
   const bool occupied = valid && cnt > 0;
 
   // refine, one direction at a time; the move is cen + sum(w e) / sum(w)
   uint32_t mask = 0;
-  double swd = 0, sxd[2] = {0, 0};
   float swf = 0.f, sxf[2] = {0.f, 0.f};
 #pragma unroll 1
   for (int k = 0; k < Q; ++k) {
@@ -285,15 +272,9 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
             real w;
             if constexpr (LOCAL) w = s_w[m];
             else w = exp(fstar_at<Q, 2, P>(A, (uint32_t)m, k));
-            if constexpr (F64) {
-              swd = __dadd_rn(swd, w);
-              sxd[0] = __dadd_rn(sxd[0], __dmul_rn(w, e[0]));
-              sxd[1] = __dadd_rn(sxd[1], __dmul_rn(w, e[1]));
-            } else {
-              swf += w;
-              sxf[0] = fmaf(w, e[0], sxf[0]);
-              sxf[1] = fmaf(w, e[1], sxf[1]);
-            }
+            swf += w;
+            sxf[0] = fmaf(w, e[0], sxf[0]);
+            sxf[1] = fmaf(w, e[1], sxf[1]);
           }
         }
       }
@@ -314,7 +295,6 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
     if (kappa <= A.kappa_hard) np[a] = cen[a];
-    else if constexpr (F64) np[a] = __dadd_rn(cen[a], __ddiv_rn(sxd[a], swd));
     else np[a] = cen[a] + sxf[a] / swf;
   }
   bool finite = true;
@@ -463,7 +443,6 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
                                                  const Item<typename P::real>* s_it, const typename P::real* s_w,
                                                  int cap) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int lx = threadIdx.x % G.tx, ly = threadIdx.x / G.tx;
   const int Fx = T.x0 + lx, Fy = T.y0 + ly;
   if (ly >= G.ty || Fx >= I.dims[0] || Fy >= I.dims[1]) return;
@@ -473,7 +452,6 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
 
   // thinning
   uint32_t cnt = 0;
-  real sum[2] = {0, 0};
   CSum csum[2];
 #pragma unroll 1
   for (int k = 0; k < Q; ++k) {
@@ -494,13 +472,8 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
         if (tx >= -sxf && tx < (real)1 - sxf && ty >= fy0 && ty < fy0 + (real)1) {
           ++cnt;
           const real rx = rn_add(sxf, tx), ry = rn_add(sy, ty);
-          if constexpr (F64) {
-            sum[0] += rx;
-            sum[1] += ry;
-          } else {
-            csum[0].add(rx);
-            csum[1].add(ry);
-          }
+          csum[0].add(rx);
+          csum[1].add(ry);
         }
       }
     }
@@ -515,20 +488,13 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
     return;
   }
   real cen[2];
-  if constexpr (F64) {
-    cen[0] = sum[0] / (real)cnt;
-    cen[1] = sum[1] / (real)cnt;
-  } else {
-    cen[0] = csum[0].value() / (real)cnt;
-    cen[1] = csum[1].value() / (real)cnt;
-  }
+  cen[0] = csum[0].value() / (real)cnt;
+  cen[1] = csum[1].value() / (real)cnt;
 
   // refine
   uint32_t mask = 0;
-  double swd = 0, sxd[2] = {0, 0};
   float swf = 0.f, sxf[2] = {0.f, 0.f};
   if constexpr (SHIFT) {
-    static_assert(!F64, "the shifted windows serve the FP32 store");
     refine_shift<Q, kShiftRows>(A, rw, rh, s_beg, s_end, s_it, s_w, cap, bx, by, Pair<float>{cen[0], cen[1]}, mask, swf, sxf);
   } else {
 #pragma unroll 1
@@ -566,15 +532,9 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
         if (d2 <= A.R2) {
           mask |= 1u << k;
           const real w = wk[m];
-          if constexpr (F64) {
-            swd = __dadd_rn(swd, w);
-            sxd[0] = __dadd_rn(sxd[0], __dmul_rn(w, ex));
-            sxd[1] = __dadd_rn(sxd[1], __dmul_rn(w, ey));
-          } else {
-            swf += w;
-            sxf[0] = fmaf(w, ex, sxf[0]);
-            sxf[1] = fmaf(w, ey, sxf[1]);
-          }
+          swf += w;
+          sxf[0] = fmaf(w, ex, sxf[0]);
+          sxf[1] = fmaf(w, ey, sxf[1]);
         }
       }
     }
@@ -585,7 +545,6 @@ __device__ __forceinline__ void thin_refine_rows(const Args<Q, 2, P>& A, const I
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
     if (kappa <= A.kappa_hard) np[a] = cen[a];
-    else if constexpr (F64) np[a] = __dadd_rn(cen[a], __ddiv_rn(sxd[a], swd));
     else np[a] = cen[a] + sxf[a] / swf;
   }
   bool finite = true;
@@ -722,7 +681,6 @@ __device__ __forceinline__ void weights_body(const Args<Q, 2, P>& A, const InstK
                                              const Pair<typename P::real>* s_cpos, int* s_tr, int* s_ij, short* s_bx,
                                              short* s_by, Pair<typename P::real>* s_mpos) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int cap_t = G.cap_tile;
   const real* gpx = A.b.off;
   const real* gpy = A.b.off + A.ccap;
@@ -744,7 +702,6 @@ __device__ __forceinline__ void weights_body(const Args<Q, 2, P>& A, const InstK
         const real tx = rn_add(o[0], cdx), ty = rn_add(o[1], cdy);
         const int lox = max((int)floor(tx - A.R - A.tiny), -bx), hix = min((int)floor(tx + A.R + A.tiny), rw - 1 - bx);
         const int loy = max((int)floor(ty - A.R - A.tiny), -by), hiy = min((int)floor(ty + A.R + A.tiny), rh - 1 - by);
-        double swd = 0;
         CSum sws;
         bool more = false;  // (2D FP32) a window cell holds a second item: a second pass takes those
 #pragma unroll 1
@@ -772,15 +729,13 @@ __device__ __forceinline__ void weights_body(const Args<Q, 2, P>& A, const InstK
               const real d2 = canon_d2<2, real>(o, cc, e);
               if (d2 <= A.R2) {
                 const real d = rn_sqrt(d2);
-                if constexpr (F64) swd += A.R - d;
-                else sws.add(A.R - d);
+                sws.add(A.R - d);
               }
             }
           }
         }
         real sw;
-        if constexpr (F64) sw = swd;
-        else sw = sws.value();
+        sw = sws.value();
         A.sw[(int64_t)k * A.mcap + s_ij[i]] = sw > (real)0 ? (real)1 / sw : (real)0;
       }
     }
@@ -795,7 +750,6 @@ __device__ __forceinline__ void weights_rows(const Args<Q, 2, P>& A, const InstK
                                              const Item<typename P::real>* s_cit, int* s_tr, int* s_ij, short* s_bx,
                                              short* s_by, Pair<typename P::real>* s_mpos) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int cap_t = G.cap_tile;
   for (int c0 = 0;; c0 += cap_t) {
     const int n = tile_items<real>(I, T, G, G.cp, A.a.start, A.a.cell, A.a.off, A.mcap, c0, cap_t, s_tr, s_ij, s_bx,
@@ -812,7 +766,6 @@ __device__ __forceinline__ void weights_rows(const Args<Q, 2, P>& A, const InstK
         const Pair<real> o = s_mpos[i];
         const real tx = rn_add(o.x, cdx), ty = rn_add(o.y, cdy);
         const int loy = max((int)floor(ty - A.R - A.tiny), -by), hiy = min((int)floor(ty + A.R + A.tiny), rh - 1 - by);
-        double swd = 0;
         CSum sws;
         bool more = false;  // (2D FP32) a window cell holds a second item: a second pass takes those
 #pragma unroll 1
@@ -845,14 +798,12 @@ __device__ __forceinline__ void weights_rows(const Args<Q, 2, P>& A, const InstK
             const real d2 = rn_add(rn_mul(ex, ex), rn_mul(ey, ey));
             if (d2 <= A.R2) {
               const real d = rn_sqrt(d2);
-              if constexpr (F64) swd += A.R - d;
-              else sws.add(A.R - d);
+              sws.add(A.R - d);
             }
           }
         }
         real sw;
-        if constexpr (F64) sw = swd;
-        else sw = sws.value();
+        sw = sws.value();
         A.sw[(int64_t)k * A.mcap + s_ij[i]] = sw > (real)0 ? (real)1 / sw : (real)0;
       }
     }
@@ -994,7 +945,6 @@ __device__ __forceinline__ void gather_body(const Args<Q, 2, P>& A, const InstK&
                                             int* s_tr, int* s_ij, short* s_bx, short* s_by,
                                             Pair<typename P::real>* s_cpos) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int cap_t = G.cap_tile;
   const real* gox = A.a.off;
   const real* goy = A.a.off + A.mcap;
@@ -1005,7 +955,7 @@ __device__ __forceinline__ void gather_body(const Args<Q, 2, P>& A, const InstK&
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
       const real* ginv = A.sw + (int64_t)k * A.mcap;
-      const real* gfk = F64 ? (const real*)(A.a.f64 + (int64_t)k * A.mcap) : (const real*)(A.a.dev + (int64_t)k * A.mcap);
+      const real* gfk = A.a.dev + (int64_t)k * A.mcap;
       if constexpr (LOCAL) {
         __syncthreads();
         for (int l = threadIdx.x; l < nstaged; l += blockDim.x) {
@@ -1021,7 +971,6 @@ __device__ __forceinline__ void gather_body(const Args<Q, 2, P>& A, const InstK&
         const real bxr = pp.x - cdx, byr = pp.y - cdy;
         const int lox = max((int)floor(bxr - A.R - A.tiny), -bx), hix = min((int)floor(bxr + A.R + A.tiny), rw - 1 - bx);
         const int loy = max((int)floor(byr - A.R - A.tiny), -by), hiy = min((int)floor(byr + A.R + A.tiny), rh - 1 - by);
-        double acc = 0;
         CSum sa;
         float sb = 0.f;  // deviation part: small, plain FMA accumulation suffices
         bool more = false;  // (2D FP32) a window cell holds a second item: a second pass takes those
@@ -1057,15 +1006,11 @@ __device__ __forceinline__ void gather_body(const Args<Q, 2, P>& A, const InstK&
                 else kv = Pair<real>{ginv[m], gfk[m]};
                 if (kv.x > (real)0) {
                   const real wgt = (A.R - rn_sqrt(d2)) * kv.x;
-                  if constexpr (F64) {
-                    acc += wgt * kv.y;
-                  } else {
-                    real rho;
-                    if constexpr (LOCAL) rho = s_rho[m];
-                    else rho = A.a.rho[m];
-                    sa.add_prod(wgt, rho);
-                    sb = __fmaf_rn(wgt, kv.y, sb);
-                  }
+                  real rho;
+                  if constexpr (LOCAL) rho = s_rho[m];
+                  else rho = A.a.rho[m];
+                  sa.add_prod(wgt, rho);
+                  sb = __fmaf_rn(wgt, kv.y, sb);
                 }
               }
             }
@@ -1073,17 +1018,12 @@ __device__ __forceinline__ void gather_body(const Args<Q, 2, P>& A, const InstK&
         }
         const int j = s_ij[i];
         bool empty;
-        if constexpr (F64) {
-          A.cpf64[(int64_t)k * A.ccap + j] = acc;
-          empty = acc < (double)A.eps;
-        } else {
-          DF Ad = df_norm(sa.hi, sa.lo);
-          DF Bd = DF{sb, 0.f};
-          DF Fv = df_add(df_mul(DF{A.L.wf[k], A.L.wlo[k]}, Ad), Bd);
-          A.cpfhi[(int64_t)k * A.ccap + j] = Fv.hi;
-          A.cpflo[(int64_t)k * A.ccap + j] = Fv.lo;
-          empty = Fv.hi < A.eps;
-        }
+        DF Ad = df_norm(sa.hi, sa.lo);
+        DF Bd = DF{sb, 0.f};
+        DF Fv = df_add(df_mul(DF{A.L.wf[k], A.L.wlo[k]}, Ad), Bd);
+        A.cpfhi[(int64_t)k * A.ccap + j] = Fv.hi;
+        A.cpflo[(int64_t)k * A.ccap + j] = Fv.lo;
+        empty = Fv.hi < A.eps;
         if (empty) atomicOr(A.emask + j, 1u << k);
       }
     }
@@ -1100,7 +1040,6 @@ __device__ __forceinline__ void gather_rows(const Args<Q, 2, P>& A, const InstK&
                                             int* s_tr, int* s_ij, short* s_bx, short* s_by,
                                             Pair<typename P::real>* s_cpos) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int cap_t = G.cap_tile;
   for (int c0 = 0;; c0 += cap_t) {
     const int n = tile_items<real>(I, T, G, G.mom, A.b.start, A.b.cell, A.b.off, A.ccap, c0, cap_t, s_tr, s_ij, s_bx,
@@ -1109,7 +1048,7 @@ __device__ __forceinline__ void gather_rows(const Args<Q, 2, P>& A, const InstK&
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
       const real* ginv = A.sw + (int64_t)k * A.mcap;
-      const real* gfk = F64 ? (const real*)(A.a.f64 + (int64_t)k * A.mcap) : (const real*)(A.a.dev + (int64_t)k * A.mcap);
+      const real* gfk = A.a.dev + (int64_t)k * A.mcap;
       // stage (1/sw, f_k) of every region item for this direction
       __syncthreads();
       for (int l = threadIdx.x; l < nstaged; l += blockDim.x) {
@@ -1124,7 +1063,6 @@ __device__ __forceinline__ void gather_rows(const Args<Q, 2, P>& A, const InstK&
         const Pair<real> pp = s_cpos[i];
         const real bxr = pp.x - cdx, byr = pp.y - cdy;
         const int loy = max((int)floor(byr - A.R - A.tiny), -by), hiy = min((int)floor(byr + A.R + A.tiny), rh - 1 - by);
-        double acc = 0;
         CSum sa;
         float sb = 0.f;  // deviation part: small, plain FMA accumulation suffices
         bool more = false;  // (2D FP32) a window cell holds a second item: a second pass takes those
@@ -1157,29 +1095,20 @@ __device__ __forceinline__ void gather_rows(const Args<Q, 2, P>& A, const InstK&
               const Pair<real> kv = s_kv[m];
               if (kv.x > (real)0) {
                 const real wgt = (A.R - rn_sqrt(d2)) * kv.x;
-                if constexpr (F64) {
-                  acc += wgt * kv.y;
-                } else {
-                  sa.add_prod(wgt, s_rho[m]);
-                  sb = __fmaf_rn(wgt, kv.y, sb);
-                }
+                sa.add_prod(wgt, s_rho[m]);
+                sb = __fmaf_rn(wgt, kv.y, sb);
               }
             }
           }
         }
         const int j = s_ij[i];
         bool empty;
-        if constexpr (F64) {
-          A.cpf64[(int64_t)k * A.ccap + j] = acc;
-          empty = acc < (double)A.eps;
-        } else {
-          DF Ad = df_norm(sa.hi, sa.lo);
-          DF Bd = DF{sb, 0.f};
-          DF Fv = df_add(df_mul(DF{A.L.wf[k], A.L.wlo[k]}, Ad), Bd);
-          A.cpfhi[(int64_t)k * A.ccap + j] = Fv.hi;
-          A.cpflo[(int64_t)k * A.ccap + j] = Fv.lo;
-          empty = Fv.hi < A.eps;
-        }
+        DF Ad = df_norm(sa.hi, sa.lo);
+        DF Bd = DF{sb, 0.f};
+        DF Fv = df_add(df_mul(DF{A.L.wf[k], A.L.wlo[k]}, Ad), Bd);
+        A.cpfhi[(int64_t)k * A.ccap + j] = Fv.hi;
+        A.cpflo[(int64_t)k * A.ccap + j] = Fv.lo;
+        empty = Fv.hi < A.eps;
         if (empty) atomicOr(A.emask + j, 1u << k);
       }
     }
@@ -1357,7 +1286,6 @@ template <int Q, class P>
 __device__ __forceinline__ void gather_tile(const Args<Q, 2, P>& A, const Tile2& T, const InstK& I, const TileGeo& G,
                                             unsigned char* smem) {
   using real = typename P::real;
-  constexpr bool F64 = std::is_same<P, PF64>::value;
   const int rw = G.tx + G.mom.xh - G.mom.xl, rh = G.ty + G.mom.yh - G.mom.yl;
   const int cap = G.cap_gather, cap_t = G.cap_tile;
   unsigned char* p = smem;
@@ -1377,7 +1305,7 @@ __device__ __forceinline__ void gather_tile(const Args<Q, 2, P>& A, const Tile2&
                [&](int gm, int l, int rx) {
                  s_gi[l] = gm;
                  s_it[l] = Item<real>{A.a.off[gm], A.a.off[A.mcap + gm], (real)rx, (real)0};
-                 if constexpr (!F64) s_rho[l] = A.a.rho[gm];
+                 s_rho[l] = A.a.rho[gm];
                });
   if (s_row[rh + 1])
     gather_rows<Q, P>(A, I, T, G, rw, rh, s_beg, s_end, s_gi, s_it, s_rho, s_kv, s_row[rh], s_tr, s_ij, s_bx, s_by,
