@@ -3,15 +3,16 @@
 // These keep the data layout of direbm/warp/propagation.py (positions (N,2), values (N,),
 // directions (N,), moments (M,Q) row-major) so the drop-in Python module can hand them numpy
 // arrays the way the reference tests do.  Components here are arbitrary points in an unbounded
-// plane, so neighbour queries use a sorted-cell index: points sorted by a 64-bit (x-cell,
-// y-cell) key, unique cells found by head flags + compaction, and a query binary-searches the
-// unique keys of the 5x5 cells around it (a radius-dx disc spans at most 3x3 cells; the extra ring
-// covers FP32 rounding of x/dx at cell borders -- the distance test decides).
+// plane, so neighbour queries use a sorted-cell index: the points' bounds are read back first, so that
+// the cell keys are as short as the points allow (16 bits in place of 64 for 192 x 192 cells, two radix
+// passes in place of eight) and, where the box is not mostly empty, a table of cell starts takes the place
+// of binary searches.  The cells of one x column that a query needs are consecutive: one run of items.
 //
 // The radius test is |a - b| with round-to-nearest FP32 steps and no fused multiply-add, so the
 // pairs found are the oracle's (oracle/stages.py) bit for bit.  Sums run in a fixed order per
 // thread with compensated accumulators: there are no float atomics and results are reproducible.
 #include <algorithm>
+#include <mutex>
 
 #include "lattice.cuh"
 #include "sortscan.cuh"
@@ -23,8 +24,13 @@ __device__ __forceinline__ float dist32(float ax, float ay, float bx, float by) 
   return __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
 }
 
-__device__ __forceinline__ uint64_t pack_cell(long long ix, long long iy) {
-  return ((uint64_t)(uint32_t)(ix + 2147483648LL) << 32) | (uint64_t)(uint32_t)(iy + 2147483648LL);
+// Points of the caller's arrays: 4-byte aligned, no wider loads.
+__device__ __forceinline__ float2 load2(const float* __restrict__ p, int64_t i) {
+  return make_float2(p[2 * i], p[2 * i + 1]);
+}
+__device__ __forceinline__ void store2(float* __restrict__ p, int64_t i, float2 v) {
+  p[2 * i] = v.x;
+  p[2 * i + 1] = v.y;
 }
 
 __device__ __forceinline__ long long cell_of(float x, float cs) { return (long long)floorf(__fdiv_rn(x, cs)); }
@@ -46,12 +52,118 @@ __global__ void k_disperse(const float* __restrict__ pos_m, const float* __restr
   }
 }
 
-__global__ void k_keys(const float* __restrict__ pos, int64_t n, float cs, uint64_t* __restrict__ keys,
-                       uint32_t* __restrict__ vals) {
+// Cells as 32-bit words whose order is the cells'.
+__device__ __forceinline__ uint32_t cell_word(long long i) { return (uint32_t)((unsigned long long)i + 2147483648ULL); }
+
+// Bounds of the points' cells: (min x, min y, ~max x, ~max y), all set to ones before.
+__global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ pos, int64_t n, float cs,
+                                                uint32_t* __restrict__ bounds) {
+  uint32_t lo[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    keys[i] = pack_cell(cell_of(pos[2 * i], cs), cell_of(pos[2 * i + 1], cs));
-    vals[i] = (uint32_t)i;
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      const uint32_t c = cell_word(cell_of(pos[2 * i + a], cs));
+      lo[a] = min(lo[a], c);
+      lo[2 + a] = min(lo[2 + a], ~c);
+    }
   }
+  __shared__ uint32_t s_lo[4];
+  if (threadIdx.x < 4) s_lo[threadIdx.x] = 0xffffffffu;
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const uint32_t w = __reduce_min_sync(0xffffffffu, lo[a]);
+    if ((threadIdx.x & 31) == 0) atomicMin(&s_lo[a], w);
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) atomicMin(&bounds[threadIdx.x], s_lo[threadIdx.x]);
+}
+
+// A sorted-cell index over n points (cell size cs).  Key of a cell: dense, dx * ny + dy from the lower
+// bounds; else dx << by | dy.
+struct PointIndex {
+  uint32_t minx = 0, miny = 0, maxx = 0xffffffffu, maxy = 0xffffffffu;
+  uint32_t ny = 0;           // dense: cells along y (0: not dense)
+  int by = 32;
+  uint32_t n = 0;
+  uint64_t* keys = nullptr;   // sorted cell keys [n]
+  uint32_t* order = nullptr;  // point index in sorted order [n]
+  uint32_t* start = nullptr;  // dense: first item of each cell [cells + 1]
+
+  __device__ __forceinline__ uint64_t key(uint32_t wx, uint32_t wy) const {
+    return ny ? (uint64_t)(wx - minx) * ny + (wy - miny) : ((uint64_t)(wx - minx) << by) | (wy - miny);
+  }
+  __device__ __forceinline__ uint32_t lower(uint64_t k) const {  // first item with a key >= k
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1);
+      if (keys[mid] < k) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  }
+  // body(j) for the items of column wx, rows [wy0, wy1], in sorted order
+  template <class F>
+  __device__ __forceinline__ void run(uint32_t wx, uint32_t wy0, uint32_t wy1, F&& body) const {
+    wy0 = max(wy0, miny);
+    wy1 = min(wy1, maxy);
+    if (wy0 > wy1) return;
+    const uint64_t k0 = key(wx, wy0), k1 = k0 + (wy1 - wy0);
+    if (ny) {
+      const uint32_t e = start[k1 + 1];
+      for (uint32_t j = start[k0]; j < e; ++j) body(j);
+    } else {
+      for (uint32_t j = lower(k0); j < n && keys[j] <= k1; ++j) body(j);
+    }
+  }
+};
+
+// Cells along one axis within 1 + m of the quotient f, m above the rounding of the quotients and of the
+// distance (relative 2^-22), at most two away; from 2^40 on, where floats lie further apart than dx, its own.
+__device__ __forceinline__ void near_cells(float f, long long* lo, long long* hi) {
+  const long long c = (long long)floorf(f);
+  *lo = *hi = c;
+  if (fabsf(f) < 1.0995116e12f) {
+    const float m = 1.f + 1e-6f * (2.f + fabsf(f));
+    *lo = max((long long)floorf(f - m), c - 2);
+    *hi = min((long long)floorf(f + m), c + 2);
+  }
+}
+
+// body(j) for every item of ix that may lie within dx (its cell size) of (x, y), columns ascending, then
+// rows: three columns of three rows but for a query at a cell's edge.
+template <class F>
+__device__ __forceinline__ void near_points(const PointIndex& ix, float x, float y, float dx, F&& body) {
+  const float fx = __fdiv_rn(x, dx), fy = __fdiv_rn(y, dx);
+  if (!isfinite(fx) || !isfinite(fy) || ix.n == 0) return;  // at no finite distance from any point
+  long long x0, x1, y0, y1;
+  near_cells(fx, &x0, &x1);
+  near_cells(fy, &y0, &y1);
+  const uint32_t wy0 = cell_word(y0), wy1 = cell_word(y1);
+  for (long long c = x0;; ++c) {
+    const uint32_t wx = cell_word(c);
+    if (wx >= ix.minx && wx <= ix.maxx) {
+      if (wy0 <= wy1) {
+        ix.run(wx, wy0, wy1, body);
+      } else {  // the rows wrap around the word
+        ix.run(wx, wy0, 0xffffffffu, body);
+        ix.run(wx, 0u, wy1, body);
+      }
+    }
+    if (c == x1) break;
+  }
+}
+
+__global__ void k_keys(const float* __restrict__ pos, int64_t n, float cs, PointIndex ix) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    ix.keys[i] = ix.key(cell_word(cell_of(pos[2 * i], cs)), cell_word(cell_of(pos[2 * i + 1], cs)));
+    ix.order[i] = (uint32_t)i;
+  }
+}
+
+// One search per cell: a walk over the keys would leave a long gap between two clusters to one thread.
+__global__ void k_cell_starts(PointIndex ix, int64_t ncells) {
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c <= ncells; c += (int64_t)gridDim.x * blockDim.x)
+    ix.start[c] = ix.lower((uint64_t)c);
 }
 
 __global__ void k_heads(const uint64_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ flags) {
@@ -59,283 +171,299 @@ __global__ void k_heads(const uint64_t* __restrict__ keys, int64_t n, uint32_t* 
     flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u;
 }
 
-// unique keys and run starts from the head positions; ustart[nu] = n
-__global__ void k_runs(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ head_idx, const uint32_t* d_nu,
-                       int64_t n, uint64_t* __restrict__ ukeys, uint32_t* __restrict__ ustart) {
-  const uint32_t nu = *d_nu;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= nu; r += gridDim.x * blockDim.x) {
-    if (r < nu) {
-      ukeys[r] = keys[head_idx[r]];
-      ustart[r] = head_idx[r];
-    } else {
-      ustart[r] = (uint32_t)n;
-    }
-  }
-}
-
-// Sequential FP32 centroid per run, in sorted order (propagation.py:54-68).
-__global__ void k_centroid(const float* __restrict__ pos_c, const uint32_t* __restrict__ order,
-                           const uint32_t* __restrict__ ustart, const uint32_t* d_nu, float* __restrict__ cp) {
-  const uint32_t nu = *d_nu;
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nu; r += gridDim.x * blockDim.x) {
-    const uint32_t s = ustart[r], e = ustart[r + 1];
+// Sequential FP32 centroid per run, in sorted order (propagation.py:54-68); rank: heads before an item.
+__global__ void k_centroid(const float* __restrict__ pos_c, PointIndex ix, const uint32_t* __restrict__ rank,
+                           float* __restrict__ cp) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ix.n; i += gridDim.x * blockDim.x) {
+    const uint64_t key = ix.keys[i];
+    if (i > 0 && ix.keys[i - 1] == key) continue;
     float sx = 0.f, sy = 0.f;
-    for (uint32_t j = s; j < e; ++j) {
-      const uint32_t c = order[j];
-      sx = __fadd_rn(sx, pos_c[2 * c]);
-      sy = __fadd_rn(sy, pos_c[2 * c + 1]);
-    }
-    const float n = (float)(e - s);
-    cp[2 * r] = __fdiv_rn(sx, n);
-    cp[2 * r + 1] = __fdiv_rn(sy, n);
+    uint32_t j = i;
+    do {
+      const float2 q = load2(pos_c, ix.order[j]);
+      sx = __fadd_rn(sx, q.x);
+      sy = __fadd_rn(sy, q.y);
+    } while (++j < ix.n && ix.keys[j] == key);
+    const float n = (float)(j - i);
+    store2(cp, rank[i], make_float2(__fdiv_rn(sx, n), __fdiv_rn(sy, n)));
   }
 }
 
-// A sorted-cell index over n points (cell size cs).
-struct PointIndex {
-  uint64_t* keys = nullptr;   // sorted cell keys [n]
-  uint32_t* order = nullptr;  // point index in sorted order [n]
-  uint64_t* ukeys = nullptr;  // unique keys [n]
-  uint32_t* ustart = nullptr; // [n + 1]
-  uint32_t* nu = nullptr;     // device count of unique keys
-};
+// The temporaries' own stream-ordered pool, one per device.  Up to 64 MB stay with it between calls: the
+// default pool gives every page back at each synchronisation and maps it again on the next call.
+constexpr uint64_t kPoolKeep = 64ull << 20;
+static int stage_pool(cudaMemPool_t* out) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  DBM_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) { set_last_error("device %d: out of range", dev); return DBM_ERR_STATE; }
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    DBM_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = kPoolKeep;
+    DBM_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    pools[dev] = pool;
+  }
+  *out = pools[dev];
+  return DBM_OK;
+}
 
-struct Arena {  // stream-ordered temporaries, freed together
-  static constexpr int kMax = 64;
+// Stream-ordered temporaries of one call, cut from one allocation (`bytes`: an upper bound of their sum).
+struct Arena {
   cudaStream_t s;
-  void* ptrs[kMax];
-  int n = 0;
-  explicit Arena(cudaStream_t st) : s(st) {}
+  char* base = nullptr;
+  size_t used = 0, bytes;
+  Arena(cudaStream_t st, size_t b) : s(st), bytes(b) {}
   template <class T>
   int get(T** p, int64_t count) {
-    if (n >= kMax) {
-      set_last_error("internal: more than %d temporaries in one stage call", kMax);
-      return DBM_ERR_STATE;
+    if (!base) {
+      cudaMemPool_t pool = nullptr;
+      DBM_TRY(stage_pool(&pool));
+      void* q = nullptr;
+      const cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, pool, s);
+      if (e != cudaSuccess) { set_last_error("cudaMallocFromPoolAsync: %s", cudaGetErrorString(e)); return DBM_ERR_CUDA; }
+      base = (char*)q;
     }
-    void* q = nullptr;
-    cudaError_t e = cudaMallocAsync(&q, (size_t)std::max<int64_t>(count, 1) * sizeof(T), s);
-    if (e != cudaSuccess) { set_last_error("cudaMallocAsync: %s", cudaGetErrorString(e)); return DBM_ERR_CUDA; }
-    ptrs[n++] = q;
-    *p = (T*)q;
+    const size_t sz = ((size_t)std::max<int64_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    if (sz > bytes - used) { set_last_error("internal: a stage call's temporaries exceed their bound"); return DBM_ERR_STATE; }
+    *p = (T*)(base + used);
+    used += sz;
     return DBM_OK;
   }
   ~Arena() {
-    for (int i = 0; i < n; ++i) cudaFreeAsync(ptrs[i], s);
+    if (base) cudaFreeAsync(base, s);
   }
 };
 
+// The most cells of a table of starts for n points, and the bytes of an index with its packed items.
+static uint64_t max_cells(int64_t n) { return 4 * (uint64_t)n + 65536; }
+static size_t index_bytes(int64_t n, bool starts) {
+  const size_t m = (size_t)std::max<int64_t>(n, 1);
+  return m * (8 + 4 + 8 + 4 + 16 + 4) + radix_tmp_bytes(n) + (starts ? (size_t)(max_cells(n) + 1) * 4 : scan_tmp_bytes(n)) +
+         12 * 256;
+}
+
 static unsigned grid_for(int64_t n) { return std::min<unsigned>(div_up(std::max<int64_t>(n, 1), 256), (unsigned)sm_count() * 16); }
 
-static int build_index(const float* pos, int64_t n, float cs, Arena& ar, PointIndex* ix) {
+static int bit_length(uint64_t v) {
+  int b = 0;
+  while (b < 64 && (v >> b)) ++b;
+  return b;
+}
+
+// Bounds of one or two point sets (n > 0) on the host; false while the stream is being captured, which
+// allows no read-back.
+struct PointSet {
+  const float* pos;
+  int64_t n;
+  float cs;
+};
+static int read_bounds(const PointSet* sets, int nsets, Arena& ar, uint32_t (*bounds)[4], bool* known) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  DBM_CUDA(cudaStreamIsCapturing(ar.s, &cap));
+  *known = cap == cudaStreamCaptureStatusNone;
+  if (!*known) return DBM_OK;
+  uint32_t* d = nullptr;
+  DBM_TRY(ar.get(&d, 4 * nsets));
+  DBM_CUDA(cudaMemsetAsync(d, 0xff, (size_t)nsets * 16, ar.s));
+  for (int i = 0; i < nsets; ++i) {
+    const unsigned g = std::min<unsigned>(div_up(sets[i].n, 1024), (unsigned)sm_count() * 2);
+    k_bounds<<<g, 256, 0, ar.s>>>(sets[i].pos, sets[i].n, sets[i].cs, d + 4 * i);
+    DBM_LAUNCH_CHECK();
+  }
+  DBM_CUDA(cudaMemcpyAsync(bounds, d, (size_t)nsets * 16, cudaMemcpyDeviceToHost, ar.s));
+  DBM_CUDA(cudaStreamSynchronize(ar.s));
+  return DBM_OK;
+}
+
+// starts: the index serves neighbour queries (else only its order is used).
+static int build_index(const PointSet& p, const uint32_t (&bounds)[4], bool known, bool starts, Arena& ar,
+                       PointIndex* ix) {
   cudaStream_t s = ar.s;
-  uint64_t *k_alt;
-  uint32_t *v_alt, *flags, *heads, *dummy;
-  void* rtmp;
-  void* ctmp;
+  const int64_t n = p.n;
+  uint64_t* k_alt;
+  uint32_t* v_alt;
+  char* rtmp;
   DBM_TRY(ar.get(&ix->keys, n));
   DBM_TRY(ar.get(&ix->order, n));
   DBM_TRY(ar.get(&k_alt, n));
   DBM_TRY(ar.get(&v_alt, n));
-  DBM_TRY(ar.get(&flags, n));
-  DBM_TRY(ar.get(&heads, n));
-  DBM_TRY(ar.get(&dummy, n));
-  DBM_TRY(ar.get(&ix->ukeys, n));
-  DBM_TRY(ar.get(&ix->ustart, n + 1));
-  DBM_TRY(ar.get(&ix->nu, 1));
-  DBM_TRY(ar.get((char**)&rtmp, (int64_t)radix_tmp_bytes(n)));
-  DBM_TRY(ar.get((char**)&ctmp, (int64_t)compact_tmp_bytes(n)));
-  k_keys<<<grid_for(n), 256, 0, s>>>(pos, n, cs, ix->keys, ix->order);
+  DBM_TRY(ar.get(&rtmp, (int64_t)radix_tmp_bytes(n)));
+  ix->n = (uint32_t)n;
+  int bits = 64;
+  uint64_t cells = 0;
+  if (known) {
+    ix->minx = bounds[0];
+    ix->miny = bounds[1];
+    ix->maxx = ~bounds[2];
+    ix->maxy = ~bounds[3];
+    const uint64_t nx = (uint64_t)(ix->maxx - ix->minx) + 1, ny = (uint64_t)(ix->maxy - ix->miny) + 1;
+    ix->by = bit_length(ny - 1);
+    bits = bit_length(nx - 1) + ix->by;
+    // a table of at most four cells per point (plus a little): mostly empty boxes are searched instead
+    if (nx < (1u << 31) && ny < (1u << 31) && nx * ny <= max_cells(n)) {
+      cells = nx * ny;
+      ix->ny = (uint32_t)ny;
+      bits = bit_length(cells - 1);
+    }
+  }
+  k_keys<<<grid_for(n), 256, 0, s>>>(p.pos, n, p.cs, *ix);
   DBM_LAUNCH_CHECK();
   bool alt = false;
-  DBM_TRY(radix_sort_pairs<uint64_t>(ix->keys, ix->order, k_alt, v_alt, n, nullptr, 64, rtmp, s, &alt));
+  DBM_TRY(radix_sort_pairs<uint64_t>(ix->keys, ix->order, k_alt, v_alt, n, nullptr, bits, rtmp, s, &alt));
   if (alt) {
     ix->keys = k_alt;
     ix->order = v_alt;
   }
-  k_heads<<<grid_for(n), 256, 0, s>>>(ix->keys, n, flags);
-  DBM_LAUNCH_CHECK();
-  DBM_TRY(compact_flags_u32(flags, flags, dummy, heads, n, ix->nu, ctmp, s));
-  k_runs<<<grid_for(n + 1), 256, 0, s>>>(ix->keys, heads, ix->nu, n, ix->ukeys, ix->ustart);
-  DBM_LAUNCH_CHECK();
+  if (ix->ny && starts) {
+    DBM_TRY(ar.get(&ix->start, (int64_t)cells + 1));
+    k_cell_starts<<<grid_for((int64_t)cells + 1), 256, 0, s>>>(*ix, (int64_t)cells);
+    DBM_LAUNCH_CHECK();
+  }
   return DBM_OK;
 }
 
-__device__ __forceinline__ bool find_cell(const PointIndex& ix, uint64_t key, uint32_t* b, uint32_t* e) {
-  uint32_t lo = 0, hi = *ix.nu;
-  while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (ix.ukeys[mid] < key) lo = mid + 1; else hi = mid;
+// Components in index order: position, value (expf of it for the refine), direction or weight sum.
+__global__ void k_pack_comps(const float* __restrict__ pos_c, const float* __restrict__ val_c,
+                             const int32_t* __restrict__ dir_c, PointIndex ix, int as_weight,
+                             float4* __restrict__ items) {
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < ix.n; j += gridDim.x * blockDim.x) {
+    const uint32_t c = ix.order[j];
+    const float2 q = load2(pos_c, c);
+    const float v = val_c[c];
+    items[j] = make_float4(q.x, q.y, as_weight ? expf(v) : v, __int_as_float(dir_c[c]));
   }
-  if (lo < *ix.nu && ix.ukeys[lo] == key) {
-    *b = ix.ustart[lo];
-    *e = ix.ustart[lo + 1];
-    return true;
-  }
-  return false;
+}
+__global__ void k_pack_points(const float* __restrict__ pos, PointIndex ix, float2* __restrict__ items) {
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < ix.n; j += gridDim.x * blockDim.x)
+    items[j] = load2(pos, ix.order[j]);
 }
 
-__global__ void k_refine(const float* __restrict__ cp, int64_t p, const float* __restrict__ pos_c,
-                         const float* __restrict__ val_c, const int32_t* __restrict__ dir_c, PointIndex ix, float dx,
-                         int kappa_hard, float* __restrict__ out) {
+// 205 k points, 258 k components: 200 -> 40 us (a search per cell took 16 dependent loads, 25 times).
+__global__ void k_refine(const float* __restrict__ cp, int64_t p, const float4* __restrict__ items, PointIndex ix,
+                         float dx, int kappa_hard, float* __restrict__ out) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < p; r += (int64_t)gridDim.x * blockDim.x) {
-    const float px = cp[2 * r], py = cp[2 * r + 1];
-    const long long cx = cell_of(px, dx), cy = cell_of(py, dx);
+    const float2 q = load2(cp, r);
     uint32_t mask = 0;
     CSum sw, sx, sy;
-    for (int ox = -2; ox <= 2; ++ox)
-      for (int oy = -2; oy <= 2; ++oy) {
-        uint32_t b, e;
-        if (!find_cell(ix, pack_cell(cx + ox, cy + oy), &b, &e)) continue;
-        for (uint32_t j = b; j < e; ++j) {
-          const uint32_t c = ix.order[j];
-          const float qx = pos_c[2 * c], qy = pos_c[2 * c + 1];
-          if (dist32(qx, qy, px, py) <= dx) {
-            mask |= 1u << dir_c[c];
-            const float w = expf(val_c[c]);
-            sw.add(w);
-            sx.add_prod(w, qx);
-            sy.add_prod(w, qy);
-          }
-        }
+    near_points(ix, q.x, q.y, dx, [&](uint32_t j) {
+      const float4 it = items[j];
+      if (dist32(it.x, it.y, q.x, q.y) <= dx) {
+        mask |= 1u << __float_as_int(it.w);
+        sw.add(it.z);
+        sx.add_prod(it.z, it.x);
+        sy.add_prod(it.z, it.y);
       }
-    const int kappa = __popc(mask);
-    if (kappa <= kappa_hard) {
-      out[2 * r] = px;
-      out[2 * r + 1] = py;
+    });
+    if (__popc(mask) <= kappa_hard) {
+      store2(out, r, q);
     } else {
       const float s = sw.value();
-      out[2 * r] = sx.value() / s;
-      out[2 * r + 1] = sy.value() / s;
+      store2(out, r, make_float2(sx.value() / s, sy.value() / s));
     }
   }
 }
 
-// Pass 1 of the resampling gather: sw per component over the control points within dx.
-__global__ void k_comp_sw(const float* __restrict__ pos_c, int64_t nc, const float* __restrict__ cp, PointIndex cpi,
+// Resampling, first walk: the weight sum of each component over the control points within dx (166 -> 25 us).
+__global__ void k_comp_sw(const float4* __restrict__ comps, uint32_t nc, const float2* __restrict__ cps, PointIndex cpi,
                           float dx, float* __restrict__ sw_out) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
-    const float qx = pos_c[2 * c], qy = pos_c[2 * c + 1];
-    const long long cx = cell_of(qx, dx), cy = cell_of(qy, dx);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
+    const float4 q = comps[i];
     CSum sw;
-    for (int ox = -2; ox <= 2; ++ox)
-      for (int oy = -2; oy <= 2; ++oy) {
-        uint32_t b, e;
-        if (!find_cell(cpi, pack_cell(cx + ox, cy + oy), &b, &e)) continue;
-        for (uint32_t j = b; j < e; ++j) {
-          const uint32_t r = cpi.order[j];
-          const float d = dist32(cp[2 * r], cp[2 * r + 1], qx, qy);
-          if (d <= dx) sw.add(__fsub_rn(dx, d));
-        }
-      }
-    sw_out[c] = sw.value();
+    near_points(cpi, q.x, q.y, dx, [&](uint32_t j) {
+      const float2 c = cps[j];
+      const float d = dist32(c.x, c.y, q.x, q.y);
+      if (d <= dx) sw.add(__fsub_rn(dx, d));
+    });
+    sw_out[i] = sw.value();
   }
 }
 
-// Pass 2 as the reference's scatter (propagation.py:156-186), without its float atomics: every
-// component (m, k) with sw > 0 writes one record per control point r within dx, key r * Q + k and
-// value (dx - d)/sw * f, at offsets from a scan of its count (records in component order, control
-// points in index-walk order); the records are stable-sorted by key and each key's run is summed
-// by the warp-level segmented reduction (segreduce.cu).
-__global__ void k_scatter_count(const float* __restrict__ pos_c, int64_t nc, const float* __restrict__ cp,
-                                PointIndex cpi, const float* __restrict__ sw, float dx, uint32_t* __restrict__ cnt) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t n = 0;
-    if (sw[c] > 0.f) {
-      const float qx = pos_c[2 * c], qy = pos_c[2 * c + 1];
-      const long long cx = cell_of(qx, dx), cy = cell_of(qy, dx);
-      for (int ox = -2; ox <= 2; ++ox)
-        for (int oy = -2; oy <= 2; ++oy) {
-          uint32_t b, e;
-          if (!find_cell(cpi, pack_cell(cx + ox, cy + oy), &b, &e)) continue;
-          for (uint32_t j = b; j < e; ++j) {
-            const uint32_t r = cpi.order[j];
-            if (dist32(cp[2 * r], cp[2 * r + 1], qx, qy) <= dx) ++n;
-          }
-        }
-    }
-    cnt[c] = n;
-  }
-}
-
+// Second walk, in place of the reference's scatter with float atomics (propagation.py:156-186): every
+// control point gathers (dx - d)/sw * f of the components with sw > 0 within dx, direction by direction, in
+// index order.  A thread's sums lie in shared memory ([Q][256], its own column), since the direction of the
+// next component is not known; writing a record per pair, sorting and summing the records took 0.65 ms for
+// 4.6 M pairs where this takes 0.04.
 template <int Q>
-__global__ void k_scatter_write(const float* __restrict__ pos_c, int64_t nc, const float* __restrict__ val_c,
-                                const int32_t* __restrict__ dir_c, const float* __restrict__ cp, PointIndex cpi,
-                                const float* __restrict__ sw, float dx, const uint32_t* __restrict__ pos_of,
-                                uint32_t* __restrict__ keys, float* __restrict__ vals) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
-    const float s = sw[c];
-    if (!(s > 0.f)) continue;
-    const float qx = pos_c[2 * c], qy = pos_c[2 * c + 1];
-    const long long cx = cell_of(qx, dx), cy = cell_of(qy, dx);
-    const uint32_t k = (uint32_t)dir_c[c];
-    const float v = val_c[c];
-    uint32_t w = pos_of[c];
-    for (int ox = -2; ox <= 2; ++ox)
-      for (int oy = -2; oy <= 2; ++oy) {
-        uint32_t b, e;
-        if (!find_cell(cpi, pack_cell(cx + ox, cy + oy), &b, &e)) continue;
-        for (uint32_t j = b; j < e; ++j) {
-          const uint32_t r = cpi.order[j];
-          const float d = dist32(cp[2 * r], cp[2 * r + 1], qx, qy);
-          if (d <= dx) {
-            keys[w] = r * (uint32_t)Q + k;
-            vals[w] = __fmul_rn(__fdiv_rn(__fsub_rn(dx, d), s), v);
-            ++w;
-          }
-        }
+__global__ void __launch_bounds__(256) k_cp_gather(const float2* __restrict__ cps, PointIndex cpi,
+                                                   const float4* __restrict__ comps, const float* __restrict__ sw,
+                                                   PointIndex ci, float dx, float eps, uint32_t* __restrict__ emask,
+                                                   float* __restrict__ out_pos, float* __restrict__ out_f) {
+  __shared__ float s_hi[Q][256], s_lo[Q][256];
+  const int t = threadIdx.x;
+  for (uint32_t i = blockIdx.x * blockDim.x + t; i < cpi.n; i += gridDim.x * blockDim.x) {
+    const float2 p = cps[i];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) s_hi[q][t] = s_lo[q][t] = 0.f;
+    uint32_t seen = 0;
+    near_points(ci, p.x, p.y, dx, [&](uint32_t j) {
+      const float4 it = comps[j];
+      const float d = dist32(p.x, p.y, it.x, it.y);
+      if (!(d <= dx)) return;
+      const float s = sw[j];
+      const uint32_t k = (uint32_t)__float_as_int(it.w);
+      if (!(s > 0.f) || k >= (uint32_t)Q) return;
+      const float v = __fmul_rn(__fdiv_rn(__fsub_rn(dx, d), s), it.z);
+      if ((seen >> k) & 1u) {
+        CSum a;
+        a.hi = s_hi[k][t];
+        a.lo = s_lo[k][t];
+        a.add(v);
+        s_hi[k][t] = a.hi;
+        s_lo[k][t] = a.lo;
+      } else {
+        seen |= 1u << k;
+        s_hi[k][t] = v;
       }
-  }
-}
-
-// The emptiness mask of each control point from its resampled f (before the gap fill).
-template <int Q>
-__global__ void k_cp_emask(const float* __restrict__ cpf, int64_t p, float eps, uint32_t* __restrict__ emask) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < p; r += (int64_t)gridDim.x * blockDim.x) {
+    });
+    const uint32_t r = cpi.order[i];
     uint32_t em = 0;
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-      if (cpf[r * Q + q] < eps) em |= 1u << q;
-    emask[r] = em;
+    for (int q = 0; q < Q; ++q) {
+      const float v = __fadd_rn(s_hi[q][t], s_lo[q][t]);
+      if (v < eps) em |= 1u << q;
+      out_f[(int64_t)r * Q + q] = v;
+    }
+    emask[i] = em;
+    store2(out_pos, r, p);
   }
 }
 
+// Empty directions from the rest state, judged on the masks before the fill.
 template <int Q>
-__global__ void k_cp_fill(const float* __restrict__ cp, int64_t p, PointIndex cpi, const uint32_t* __restrict__ emask,
-                          const float* __restrict__ f_rest, float dx, float* __restrict__ cpf,
-                          float* __restrict__ out_pos, float* __restrict__ out_f) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < p; r += (int64_t)gridDim.x * blockDim.x) {
-    const float px = cp[2 * r], py = cp[2 * r + 1];
-    const uint32_t em = emask[r];
+__global__ void __launch_bounds__(256) k_cp_fill(const float2* __restrict__ cps, PointIndex cpi,
+                                                 const uint32_t* __restrict__ emask, const float* __restrict__ f_rest,
+                                                 float dx, float* __restrict__ out_f) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cpi.n; i += gridDim.x * blockDim.x) {
+    const uint32_t em = emask[i];
+    if (!em) continue;
+    const float2 p = cps[i];
     CSum sw[Q];
-    if (em) {
-      const long long cx = cell_of(px, dx), cy = cell_of(py, dx);
-      for (int ox = -2; ox <= 2; ++ox)
-        for (int oy = -2; oy <= 2; ++oy) {
-          uint32_t b, e;
-          if (!find_cell(cpi, pack_cell(cx + ox, cy + oy), &b, &e)) continue;
-          for (uint32_t j = b; j < e; ++j) {
-            const uint32_t o = cpi.order[j];
-            const uint32_t both = emask[o] & em;
-            if (!both) continue;
-            const float d = dist32(cp[2 * o], cp[2 * o + 1], px, py);
-            if (d <= dx) {
-              const float w = __fsub_rn(dx, d);
+    near_points(cpi, p.x, p.y, dx, [&](uint32_t j) {
+      const uint32_t both = emask[j] & em;
+      if (!both) return;
+      const float2 o = cps[j];
+      const float d = dist32(o.x, o.y, p.x, p.y);
+      if (d <= dx) {
+        const float w = __fsub_rn(dx, d);
 #pragma unroll
-              for (int q = 0; q < Q; ++q)
-                if ((both >> q) & 1u) sw[q].add(w);
-            }
-          }
-        }
-    }
+        for (int q = 0; q < Q; ++q)
+          if ((both >> q) & 1u) sw[q].add(w);
+      }
+    });
+    const uint32_t r = cpi.order[i];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      float v = cpf[r * Q + q];
       const float s = sw[q].value();
-      if (((em >> q) & 1u) && s > 0.f) v = (dx / s) * f_rest[q];
-      out_f[r * Q + q] = v;
+      if (((em >> q) & 1u) && s > 0.f) out_f[(int64_t)r * Q + q] = (dx / s) * f_rest[q];
     }
-    out_pos[2 * r] = px;
-    out_pos[2 * r + 1] = py;
   }
 }
 
@@ -384,12 +512,24 @@ int dbm_create_control_points_f32(const float* pos_c, int64_t nc, float cs, floa
   cudaStream_t s = (cudaStream_t)stream;
   uint32_t nu = 0;
   {
-    Arena ar(s);
+    Arena ar(s, index_bytes(nc, false) + 256);
     PointIndex ix;
-    DBM_TRY(build_index(pos_c, nc, cs, ar, &ix));
-    k_centroid<<<grid_for(nc), 256, 0, s>>>(pos_c, ix.order, ix.ustart, ix.nu, cp_pos);
+    const PointSet pts{pos_c, nc, cs};
+    uint32_t bounds[1][4];
+    bool known = false;
+    DBM_TRY(read_bounds(&pts, 1, ar, bounds, &known));
+    DBM_TRY(build_index(pts, bounds[0], known, false, ar, &ix));
+    uint32_t *flags, *d_nu;
+    char* stmp;
+    DBM_TRY(ar.get(&flags, nc));
+    DBM_TRY(ar.get(&d_nu, 1));
+    DBM_TRY(ar.get(&stmp, (int64_t)scan_tmp_bytes(nc)));
+    k_heads<<<grid_for(nc), 256, 0, s>>>(ix.keys, nc, flags);
     DBM_LAUNCH_CHECK();
-    DBM_CUDA(cudaMemcpyAsync(&nu, ix.nu, 4, cudaMemcpyDeviceToHost, s));
+    DBM_TRY(scan_exclusive_u32(flags, flags, nc, nullptr, d_nu, stmp, s));
+    k_centroid<<<grid_for(nc), 256, 0, s>>>(pos_c, ix, flags, cp_pos);
+    DBM_LAUNCH_CHECK();
+    DBM_CUDA(cudaMemcpyAsync(&nu, d_nu, 4, cudaMemcpyDeviceToHost, s));
   }
   DBM_CUDA(cudaStreamSynchronize(s));
   *p_out = nu;
@@ -405,15 +545,20 @@ int dbm_refine_control_points_f32(const float* cp, int64_t p, const float* pos_c
   }
   if (p == 0) return DBM_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  Arena ar(s);
+  Arena ar(s, index_bytes(nc, true) + 256);
   PointIndex ix;
+  float4* items = nullptr;
   if (nc > 0) {
-    DBM_TRY(build_index(pos_c, nc, dx, ar, &ix));
-  } else {
-    DBM_TRY(ar.get(&ix.nu, 1));
-    DBM_CUDA(cudaMemsetAsync(ix.nu, 0, 4, s));
+    const PointSet pts{pos_c, nc, dx};
+    uint32_t bounds[1][4];
+    bool known = false;
+    DBM_TRY(read_bounds(&pts, 1, ar, bounds, &known));
+    DBM_TRY(build_index(pts, bounds[0], known, true, ar, &ix));
+    DBM_TRY(ar.get(&items, nc));
+    k_pack_comps<<<grid_for(nc), 256, 0, s>>>(pos_c, val_c, dir_c, ix, 1, items);
+    DBM_LAUNCH_CHECK();
   }
-  k_refine<<<grid_for(p), 256, 0, s>>>(cp, p, pos_c, val_c, dir_c, ix, dx, kappa_hard, new_pos);
+  k_refine<<<grid_for(p), 256, 0, s>>>(cp, p, items, ix, dx, kappa_hard, new_pos);
   DBM_LAUNCH_CHECK();
   return DBM_OK;
 }
@@ -433,58 +578,33 @@ int dbm_resample_f32(const float* pos_c, const float* val_c, const int32_t* dir_
     using LT = decltype(tag);
     if constexpr (LT::D == 2) {
       constexpr int Q = LT::Q;
-      Arena ar(s);
+      Arena ar(s, index_bytes(p, true) + index_bytes(nc, true) + 256);
       PointIndex cpi, ci;
-      DBM_TRY(build_index(cp, p, dx, ar, &cpi));
-      float *sw, *cpf;
+      const PointSet sets[2] = {{cp, p, dx}, {pos_c, nc, dx}};
+      uint32_t bounds[2][4];
+      bool known = false;
+      DBM_TRY(read_bounds(sets, nc > 0 ? 2 : 1, ar, bounds, &known));
+      float2* cps;
+      float4* comps = nullptr;
+      float* sw = nullptr;
       uint32_t* em;
-      DBM_TRY(ar.get(&sw, nc));
-      DBM_TRY(ar.get(&cpf, p * Q));
+      DBM_TRY(build_index(sets[0], bounds[0], known, true, ar, &cpi));
+      DBM_TRY(ar.get(&cps, p));
       DBM_TRY(ar.get(&em, p));
-      if (nc > 0) {
-        DBM_TRY(build_index(pos_c, nc, dx, ar, &ci));
-        k_comp_sw<<<grid_for(nc), 256, 0, s>>>(pos_c, nc, cp, cpi, dx, sw);
-        DBM_LAUNCH_CHECK();
-      } else {
-        DBM_TRY(ar.get(&ci.nu, 1));
-        DBM_CUDA(cudaMemsetAsync(ci.nu, 0, 4, s));
-      }
-      DBM_CUDA(cudaMemsetAsync(cpf, 0, (size_t)p * Q * sizeof(float), s));
-      if (nc > 0) {
-        // the scatter: pair records, stable sort by (control point, direction), segmented sums
-        uint32_t *cnt, *pos_of, *d_total;
-        DBM_TRY(ar.get(&cnt, nc));
-        DBM_TRY(ar.get(&pos_of, nc));
-        DBM_TRY(ar.get(&d_total, 1));
-        char* stmp;
-        DBM_TRY(ar.get(&stmp, (int64_t)scan_tmp_bytes(nc)));
-        k_scatter_count<<<grid_for(nc), 256, 0, s>>>(pos_c, nc, cp, cpi, sw, dx, cnt);
-        DBM_LAUNCH_CHECK();
-        DBM_TRY(scan_exclusive_u32(cnt, pos_of, nc, nullptr, d_total, stmp, s));
-        uint32_t total = 0;  // the record count sizes the sort
-        DBM_CUDA(cudaMemcpyAsync(&total, d_total, 4, cudaMemcpyDeviceToHost, s));
-        DBM_CUDA(cudaStreamSynchronize(s));
-        if (total > 0) {
-          uint32_t *rk, *rv, *rk2, *rv2;
-          DBM_TRY(ar.get(&rk, total));
-          DBM_TRY(ar.get(&rv, total));
-          DBM_TRY(ar.get(&rk2, total));
-          DBM_TRY(ar.get(&rv2, total));
-          char* rtmp;
-          DBM_TRY(ar.get(&rtmp, (int64_t)radix_tmp_bytes(total)));
-          k_scatter_write<Q><<<grid_for(nc), 256, 0, s>>>(pos_c, nc, val_c, dir_c, cp, cpi, sw, dx, pos_of, rk,
-                                                         reinterpret_cast<float*>(rv));
-          DBM_LAUNCH_CHECK();
-          int bits = 1;
-          while (bits < 32 && ((uint64_t)1 << bits) < (uint64_t)p * Q) ++bits;
-          bool alt = false;  // the values travel as their bit patterns
-          DBM_TRY(radix_sort_pairs<uint32_t>(rk, rv, rk2, rv2, total, nullptr, bits, rtmp, s, &alt));
-          DBM_TRY(segmented_sum_f32(alt ? rk2 : rk, reinterpret_cast<const float*>(alt ? rv2 : rv), total, cpf, s));
-        }
-      }
-      k_cp_emask<Q><<<grid_for(p), 256, 0, s>>>(cpf, p, eps, em);
+      k_pack_points<<<grid_for(p), 256, 0, s>>>(cp, cpi, cps);
       DBM_LAUNCH_CHECK();
-      k_cp_fill<Q><<<grid_for(p), 256, 0, s>>>(cp, p, cpi, em, f_rest, dx, cpf, out_pos, out_f);
+      if (nc > 0) {
+        DBM_TRY(build_index(sets[1], bounds[1], known, true, ar, &ci));
+        DBM_TRY(ar.get(&comps, nc));
+        DBM_TRY(ar.get(&sw, nc));
+        k_pack_comps<<<grid_for(nc), 256, 0, s>>>(pos_c, val_c, dir_c, ci, 0, comps);
+        DBM_LAUNCH_CHECK();
+        k_comp_sw<<<grid_for(nc), 256, 0, s>>>(comps, (uint32_t)nc, cps, cpi, dx, sw);
+        DBM_LAUNCH_CHECK();
+      }
+      k_cp_gather<Q><<<grid_for(p), 256, 0, s>>>(cps, cpi, comps, sw, ci, dx, eps, em, out_pos, out_f);
+      DBM_LAUNCH_CHECK();
+      k_cp_fill<Q><<<grid_for(p), 256, 0, s>>>(cps, cpi, em, f_rest, dx, out_f);
       DBM_LAUNCH_CHECK();
     }
     return DBM_OK;
