@@ -18,6 +18,14 @@ from .lattices import D2Q7, D3Q19, get
 from .sim import _require_cuda, _stream
 
 
+def _edges(edges, dev):
+    """The axes' edge arrays on the device, in one copy that the host does not wait for."""
+    sizes = [len(e) for e in edges]
+    host = torch.empty(sum(sizes), dtype=torch.float64, pin_memory=True)
+    np.concatenate([np.asarray(e, np.float64) for e in edges], out=host.numpy())
+    return torch.split(host.to(dev, non_blocking=True), sizes)
+
+
 def bin_fields_device(x, f, edges_x, edges_y, lattice=D2Q7, device=None):
     """Per-bin (mass, momx, momy) as CUDA tensors of shape (ny, nx)."""
     dev = _require_cuda(device)
@@ -25,8 +33,7 @@ def bin_fields_device(x, f, edges_x, edges_y, lattice=D2Q7, device=None):
     lat = get(lattice)
     x = torch.as_tensor(x, dtype=torch.float64, device=dev).contiguous()
     f = torch.as_tensor(f, dtype=torch.float64, device=dev).contiguous()
-    ex = torch.as_tensor(np.asarray(edges_x, np.float64), device=dev)
-    ey = torch.as_tensor(np.asarray(edges_y, np.float64), device=dev)
+    ex, ey = _edges((edges_x, edges_y), dev)
     n = int(x.shape[0])
     nx, ny = len(edges_x) - 1, len(edges_y) - 1
     mass = torch.empty((ny, nx), dtype=torch.float64, device=dev)
@@ -51,7 +58,7 @@ def bin_fields3_device(x, f, edges_x, edges_y, edges_z, lattice=D3Q19, device=No
     f = torch.as_tensor(f, dtype=torch.float64, device=dev).contiguous()
     if x.ndim != 2 or x.shape[1] != 3 or f.shape != (x.shape[0], lat.Q):
         raise ValueError("bin_fields3_device: expected x (n, 3) and f (n, Q)")
-    ed = [torch.as_tensor(np.asarray(e, np.float64), device=dev) for e in (edges_x, edges_y, edges_z)]
+    ed = _edges((edges_x, edges_y, edges_z), dev)
     n = int(x.shape[0])
     shape = (len(edges_z) - 1, len(edges_y) - 1, len(edges_x) - 1)
     out = [torch.empty(shape, dtype=torch.float64, device=dev) for _ in range(4)]
