@@ -989,9 +989,11 @@ template <int Q, int D, class P>
 __global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D, P> A, int only_gaps) {
   using real = typename P::real;
   const uint32_t Pn = *A.d_P;
+  bool shared = false;  // the gather's blocks shared the directions and emitted nothing
+  if constexpr (D == 2) shared = A.share_slots && direction_shares<Q>(*A.a.count, A.share_slots) > 1;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < Pn; j += gridDim.x * blockDim.x) {
     const uint32_t em = A.emask[j];
-    if (only_gaps && !em) continue;  // emitted by the gather
+    if (only_gaps && !em && !shared) continue;  // emitted by the gather
     const uint32_t G = A.b.cell[j];
     const int b = find_instance(A.inst_base, A.n_inst, G);
     const InstK I = A.inst[b];
@@ -1452,6 +1454,8 @@ struct SimImpl : SimBase {
   size_t sm_grid[3] = {0, 0, 0};
   int pgrid_grid[3] = {1, 1, 1};
   int pgrid_ds[3] = {1, 1, 1};
+  int grid_y = 1;                 // most blocks per tile, grid kernels (weights, gather)
+  int split_ds[3] = {1, 1, 1};    // blocks per tile, dense kernels
   int* d_fb = nullptr;
   // 3D grid kernels (k_brick3): bricks of 8^3 cells away from obstacles, the other bricks (8 x 8 x 4, for
   // the untiled kernels), and per stage the bricks they defer (d_fb3[0..2] counts, [3] odd_f, + 4 list)
@@ -1961,13 +1965,19 @@ struct SimImpl : SimBase {
         const void* kf[3] = {(const void*)k_grid_fallback<Q, 0>, (const void*)k_grid_fallback<Q, 1>,
                              (const void*)k_grid_fallback<Q, 2>};
         const size_t sf[3] = {sm_refine, sm_weights, sm_gather};
+        int slots = 1 << 30;
         for (int i = 0; i < 3; ++i) {
           DBM_CUDA(cudaFuncSetAttribute(kg[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_grid[i]));
           DBM_CUDA(cudaFuncSetAttribute(kf[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf[i]));
           int nbd = 1;
           DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kg[i], 256, sm_grid[i]));
           pgrid_grid[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
+          if (i > 0) slots = std::min(slots, std::max(nbd, 1) * sm_count());
         }
+        // shares of a tile (sim_grid.cuh): none where even the idle blocks would not fit four times over
+        grid_y = (int)std::min<int64_t>(Q, (int64_t)4 * slots / std::max(ntiles, 1));
+        if (grid_y < 2) grid_y = 1;
+        args.share_slots = grid_y > 1 ? slots : 0;
       }
       if (shift_ok) {
         DBM_CUDA(cudaFuncSetAttribute((const void*)k_gather_ts<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1988,14 +1998,22 @@ struct SimImpl : SimBase {
         const void* kds[3];
         with_near([&](auto tx) {
           kds[0] = (const void*)k_thin_refine_ds<Q, tx.value>;
-          kds[1] = (const void*)k_weights_ds<Q, tx.value>;
-          kds[2] = (const void*)k_gather_ds<Q, tx.value>;
+          kds[1] = (const void*)k_weights_ds<Q, tx.value, false>;
+          kds[2] = (const void*)k_gather_ds<Q, tx.value, false>;
         });
         for (int i = 0; i < 3; ++i) {
           DBM_CUDA(cudaFuncSetAttribute(kds[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
           int nbd = 1;
           DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kds[i], 256, sm_ds[i]));
           pgrid_ds[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
+          split_ds[i] = 1;
+          if constexpr (Q == 9) {
+            if (i > 0 && near_ok && geo.tx == 32 && ntiles * 3 <= std::max(nbd, 1) * sm_count()) {
+              split_ds[i] = 3;
+              DBM_CUDA(cudaFuncSetAttribute(i == 1 ? (const void*)k_weights_ds<Q, 32, true> : (const void*)k_gather_ds<Q, 32, true>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
+            }
+          }
         }
         DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 0>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
@@ -2293,7 +2311,11 @@ struct SimImpl : SimBase {
         if (shift_ok && use_shift && use_dense) {
           const int grid = use_persistent ? pgrid_ds[1] : ntiles;
           with_near([&](auto tx) {
-            k_weights_ds<Q, tx.value><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+            if constexpr (Q == 9 && tx.value == 32)
+              if (split_ds[1] > 1)
+                return k_weights_ds<Q, 32, true><<<dim3(grid, 3), 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles,
+                                                                                      d_fb + 4, d_fb + 1);
+            k_weights_ds<Q, tx.value, false><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
           });
           DBM_LAUNCH_CHECK();
           k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
@@ -2301,7 +2323,7 @@ struct SimImpl : SimBase {
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[1] : ntiles;
           with_grid([&](auto w) {
-            k_weights_grid<Q, w.value><<<grid, 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+            k_weights_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
           });
           DBM_LAUNCH_CHECK();
           k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
@@ -2326,17 +2348,30 @@ struct SimImpl : SimBase {
     if (upto <= 4) return DBM_OK;
     // the dense gather writes every control point's empty mask and, unless the step keeps its
     // intermediates, emits the points without an empty direction itself
-    bool dense = false;
-    if constexpr (kTiles) dense = (tiled_path() && shift_ok && use_shift && use_dense) || grid_path();
-    const int fuse = (dense || brick3_path()) && !A.write_trace ? 1 : 0;
-    if (!dense) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
+    bool dense = false, split = false, shared = false;  // shared: split if the device says so
+    if constexpr (kTiles) {
+      if (tiled_path() && shift_ok && use_shift && use_dense) {
+        dense = true;
+        split = split_ds[2] > 1;
+      } else if (grid_path()) {
+        dense = true;
+        shared = grid_y > 1;
+      }
+    }
+    const int fuse = ((dense && !split) || brick3_path()) && !A.write_trace ? 1 : 0;
+    if (!dense || split || shared) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (kTiles) {
       if (tiled_path()) {
         bool shifted = false;
         if (shift_ok && use_shift && use_dense) {
           const int grid = use_persistent ? pgrid_ds[2] : ntiles;
           with_near([&](auto tx) {
-            k_gather_ds<Q, tx.value><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + 4, d_fb + 2, fuse);
+            if constexpr (Q == 9 && tx.value == 32)
+              if (split_ds[2] > 1)
+                return k_gather_ds<Q, 32, true><<<dim3(grid, 3), 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles,
+                                                                                     d_fb + 4, d_fb + 2, fuse);
+            k_gather_ds<Q, tx.value, false><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + 4, d_fb + 2,
+                                                                        fuse);
           });
           DBM_LAUNCH_CHECK();
           k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2, fuse);
@@ -2344,7 +2379,7 @@ struct SimImpl : SimBase {
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[2] : ntiles;
           with_grid([&](auto w) {
-            k_gather_grid<Q, w.value><<<grid, 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 2, fuse);
+            k_gather_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 2, fuse);
           });
           DBM_LAUNCH_CHECK();
           k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 2, fuse);

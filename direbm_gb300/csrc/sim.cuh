@@ -130,6 +130,7 @@ struct Args {
   int any_obstacle;
   uint32_t* status;
   uint32_t* d_P;
+  int share_slots;  // (grid kernels) blocks that run at once, 0: one block per tile
   int* odd_f;      // (dense kernels) set by the collision: a density is negative or an f* not finite
   int write_trace;
 };
@@ -366,6 +367,18 @@ struct SimBase {
   uint32_t n_cells = 0;
 };
 
+// Blocks that share a tile's directions in the grid kernels (sim_grid.cuh), for so many moments.
+template <int Q>
+__device__ __forceinline__ int direction_shares(uint32_t moments, int slots) {
+  const int tiles = (int)(moments / 256) + 1;
+  int shares = 1;
+#pragma unroll
+  for (int per = Q - 1; per >= 1; --per) {
+    const int n = (Q + per - 1) / per;
+    if (tiles * n <= slots) shares = n;
+  }
+  return shares;
+}
 }  // namespace dbm
 
 struct dbm_sim {

@@ -593,7 +593,7 @@ __device__ __forceinline__ void weights_ds_unit(const Args<Q, 2, PF32>& A, const
   A.sw[(int64_t)k * A.mcap + m] = sw > 0.f ? 1.f / sw : 0.f;
 }
 
-template <int Q, int TX>
+template <int Q, int TX, bool SPLIT>
 __device__ __forceinline__ bool weights_ds_tile(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
                                                 const TileGeo& G, unsigned char* smem) {
   using Lay = DenseLayoutOf<Q, 1, TX>;
@@ -628,7 +628,7 @@ __device__ __forceinline__ bool weights_ds_tile(const Args<Q, 2, PF32>& A, const
 #pragma unroll
         for (int a = 0; a < 4; ++a) bxv[a] = (float)(-(ulx + a));
 #pragma unroll 1
-        for (int cy = -1; cy <= 1; ++cy) {
+        for (int cy = SPLIT ? (int)blockIdx.y - 1 : -1; cy <= (SPLIT ? (int)blockIdx.y - 1 : 1); ++cy) {
           // the three directions (c_x, c_y), c_x = d - 1: control-point rows uly + c_y + b, and the
           // component's column a is column a + d of the six from ulx - 1
           WeightSum2 s01;
@@ -694,6 +694,7 @@ __device__ __forceinline__ bool weights_ds_tile(const Args<Q, 2, PF32>& A, const
 #pragma unroll 1
   for (int u = threadIdx.x; u < left * Q; u += blockDim.x) {
     const int q = own.index(u / Q);
+    if (SPLIT && d2q9_cy(u % Q) != (int)blockIdx.y - 1) continue;
     weights_ds_unit<Q>(A, S, no, own.item[q], u % Q, own.pos[q] & 0xffff, own.pos[q] >> 16);
   }
   return true;
@@ -792,7 +793,7 @@ __device__ __forceinline__ void emit_from_cpf(const Args<Q, D, PF32>& A, int j) 
 
 // With fuse, a control point without empty directions is emitted here (almost all are; its nine
 // sums are in registers: 72 bytes less written and read per point) and k_emit takes the others.
-template <int Q, int TX>
+template <int Q, int TX, bool SPLIT>
 __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
                                                const TileGeo& G, bool fuse, unsigned char* smem) {
   using Lay = DenseLayoutOf<Q, 2, TX>;
@@ -814,7 +815,8 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
                                          fl[fslot] = A.a.rho[m];
 #pragma unroll
                                          for (int k = 0; k < Q; ++k)
-                                           kv[k * stride + slot] = make_float2(A.sw[(int64_t)k * A.mcap + m],
+                                           if (!SPLIT || d2q9_cy(k) == (int)blockIdx.y - 1)
+                                             kv[k * stride + slot] = make_float2(A.sw[(int64_t)k * A.mcap + m],
                                                                                A.a.dev[(int64_t)k * A.mcap + m]);
                                          return 0;
                                        });
@@ -839,7 +841,7 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
         uint64_t ov6 = no ? second_item_mask(S, no, by + jly - 1, bx + jlx - 1, 6, 6) : 0u;
         DF F[Q];
 #pragma unroll 1
-        for (int cy = -1; cy <= 1; ++cy) {
+        for (int cy = SPLIT ? (int)blockIdx.y - 1 : -1; cy <= (SPLIT ? (int)blockIdx.y - 1 : 1); ++cy) {
           // the three directions (c_x, c_y), c_x = d - 1: moment rows jly - c_y + b, and the component's
           // column a is column a + 2 - d of the six from jlx - 1
           GatherSum s[3];
@@ -900,25 +902,39 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
             const int k = d == 0 ? k0 : d == 1 ? k1 : k2;
             T3[d] = gather_total(A.L.wf[k], A.L.wlo[k], s[d].hi, s[d].lo, s[d].sb);
           }
+          if constexpr (SPLIT) {
+            uint32_t empty = 0;
 #pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            if (cy < 0) F[d2q9_dir(d - 1, -1)] = T3[d];
-            else if (cy == 0) F[d2q9_dir(d - 1, 0)] = T3[d];
-            else F[d2q9_dir(d - 1, 1)] = T3[d];
+            for (int d = 0; d < 3; ++d) {
+              const int k = d == 0 ? k0 : d == 1 ? k1 : k2;
+              A.cpfhi[(int64_t)k * A.ccap + j] = T3[d].hi;
+              A.cpflo[(int64_t)k * A.ccap + j] = T3[d].lo;
+              if (T3[d].hi < A.eps) empty |= 1u << k;
+            }
+            if (empty) atomicOr(A.emask + j, empty);
+          } else {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              if (cy < 0) F[d2q9_dir(d - 1, -1)] = T3[d];
+              else if (cy == 0) F[d2q9_dir(d - 1, 0)] = T3[d];
+              else F[d2q9_dir(d - 1, 1)] = T3[d];
+            }
           }
         }
-        uint32_t empty = 0;
+        if constexpr (!SPLIT) {
+          uint32_t empty = 0;
 #pragma unroll
-        for (int k = 0; k < Q; ++k)
-          if (F[k].hi < A.eps) empty |= 1u << k;
-        A.emask[j] = empty;
-        if (fuse && !empty) {
-          emit_full<Q>(A, j, F);
-        } else {
+          for (int k = 0; k < Q; ++k)
+            if (F[k].hi < A.eps) empty |= 1u << k;
+          A.emask[j] = empty;
+          if (fuse && !empty) {
+            emit_full<Q>(A, j, F);
+          } else {
 #pragma unroll
-          for (int k = 0; k < Q; ++k) {
-            A.cpfhi[(int64_t)k * A.ccap + j] = F[k].hi;
-            A.cpflo[(int64_t)k * A.ccap + j] = F[k].lo;
+            for (int k = 0; k < Q; ++k) {
+              A.cpfhi[(int64_t)k * A.ccap + j] = F[k].hi;
+              A.cpflo[(int64_t)k * A.ccap + j] = F[k].lo;
+            }
           }
         }
       }
@@ -933,6 +949,7 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
 #pragma unroll 1
   for (int u = threadIdx.x; u < left * Q; u += blockDim.x) {
     const int e = u / Q, k = u - e * Q, q = own.index(e), i = own.item[q];
+    if (SPLIT && d2q9_cy(k) != (int)blockIdx.y - 1) continue;
     const DF F = gather_ds_unit<Q>(A, S, no, make_float2(A.b.off[i], A.b.off[A.ccap + i]), k, own.pos[q] & 0xffff,
                                    own.pos[q] >> 16);
     A.cpfhi[(int64_t)k * A.ccap + i] = F.hi;
@@ -944,8 +961,12 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
   for (int e = threadIdx.x; e < left; e += blockDim.x) {
     const uint32_t empty = own_empty[e];
     const int i = own.item[own.index(e)];
-    A.emask[i] = empty;
-    if (fuse && !empty) emit_from_cpf<Q>(A, i);
+    if constexpr (SPLIT) {
+      if (empty) atomicOr(A.emask + i, empty);
+    } else {
+      A.emask[i] = empty;
+      if (fuse && !empty) emit_from_cpf<Q>(A, i);
+    }
   }
   return true;
 }
@@ -988,7 +1009,11 @@ __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_THIN) k_thin_refine_ds(cons
   }
 }
 
-template <int Q, int TX>
+// SPLIT, for a box of few tiles: the three blocks (tile, blockIdx.y) take the directions with c_y =
+// blockIdx.y - 1, since one block per SM waits on its own loads and sums; the gather then leaves its sums
+// to the emit pass.  For as many tiles as the three blocks of each still run at once: 64 x 64 cells, ten
+// steps, 730 -> 600 us; at 256 x 256, where they would not, one block per tile is as fast.  They stage the same items and find the same fault, and the first defers the tile.
+template <int Q, int TX, bool SPLIT>
 __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_WEIGHTS) k_weights_ds(const __grid_constant__ Args<Q, 2, PF32> A,
                                                       const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
                                                       int* fb_tiles, int* fb_count) {
@@ -996,12 +1021,13 @@ __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_WEIGHTS) k_weights_ds(const
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
-    if (!weights_ds_tile<Q, TX>(A, T, I, G, smem)) defer_tile(tb, fb_tiles, fb_count);
+    if (!weights_ds_tile<Q, TX, SPLIT>(A, T, I, G, smem) && (!SPLIT || blockIdx.y == 0))
+      defer_tile(tb, fb_tiles, fb_count);
     __syncthreads();
   }
 }
 
-template <int Q, int TX>
+template <int Q, int TX, bool SPLIT>
 __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_GATHER) k_gather_ds(const __grid_constant__ Args<Q, 2, PF32> A,
                                                      const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
                                                      int* fb_tiles, int* fb_count, int fuse) {
@@ -1010,7 +1036,8 @@ __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_GATHER) k_gather_ds(const _
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
     // a negative density or an f that is not finite anywhere (noted by the collision): no dense tile
-    if (*A.odd_f || !gather_ds_tile<Q, TX>(A, T, I, G, fuse != 0, smem)) defer_tile(tb, fb_tiles, fb_count);
+    if ((*A.odd_f || !gather_ds_tile<Q, TX, SPLIT>(A, T, I, G, fuse != 0, smem)) && (!SPLIT || blockIdx.y == 0))
+      defer_tile(tb, fb_tiles, fb_count);
     __syncthreads();
   }
 }

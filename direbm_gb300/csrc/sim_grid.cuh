@@ -325,7 +325,7 @@ __device__ __forceinline__ bool thin_refine_grid_tile(const Args<Q, 2, PF32>& A,
 
 template <int Q, int W>
 __device__ __forceinline__ bool weights_grid_tile(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
-                                                  const TileGeo& G, unsigned char* smem) {
+                                                  const TileGeo& G, int shares, unsigned char* smem) {
   const GridSmem S{grid_layout(Q, 1, G), smem};
   const int s2 = S.L.s2;
   __shared__ GridOwn own;
@@ -342,6 +342,7 @@ __device__ __forceinline__ bool weights_grid_tile(const Args<Q, 2, PF32>& A, con
   }
   bool has = m1 > m;
   for (int i = m + 1; i < m1 && !many; ++i) many = own.push(i, bx, by) ? 0 : 1;
+  if (!__syncthreads_or(has)) return true;  // no moment in the tile
   if (!stage_grid<0>(I, T.x0 + G.cp.xl, T.y0 + G.cp.yl, A.b.start, A.b.off, A.ccap, S, many,
                      [&](int, float2, int, int) {}, [&](int, float2, int) {}))
     return false;
@@ -353,7 +354,7 @@ __device__ __forceinline__ bool weights_grid_tile(const Args<Q, 2, PF32>& A, con
   while (has) {
     const float2 o = make_float2(A.a.off[m], A.a.off[A.mcap + m]);
 #pragma unroll 1
-    for (int k = 0; k < Q; ++k) {
+    for (int k = blockIdx.y; k < Q; k += shares) {
       const float cdx = A.L.cdf[k][0], cdy = A.L.cdf[k][1];
       const float tx = rn_add(o.x, cdx), ty = rn_add(o.y, cdy);
       const int lox = (int)floorf(tx - A.R - A.tiny), nx = (int)floorf(tx + A.R + A.tiny) - lox + 1;
@@ -402,7 +403,7 @@ __device__ __forceinline__ void copy4_async(void* dst, const void* src) {
 // One direction's (1/sw, f*) pairs are staged while the previous direction runs (two buffers).
 template <int Q, int W>
 __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
-                                                 const TileGeo& G, bool fuse, unsigned char* smem) {
+                                                 const TileGeo& G, int shares, bool fuse, unsigned char* smem) {
   const GridSmem S{grid_layout(Q, 2, G), smem};
   const int s2 = S.L.s2, s1 = S.L.s1, n2 = S.L.n2;
   __shared__ GridOwn own;
@@ -419,6 +420,7 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
   }
   bool has = j1 > j;
   for (int i = j + 1; i < j1 && !many; ++i) many = own.push(i, bx, by) ? 0 : 1;
+  if (!__syncthreads_or(has)) return true;  // no control point in the tile
   if (!stage_grid<1>(
           I, T.x0 + G.mom.xl, T.y0 + G.mom.yl, A.a.start, A.a.off, A.mcap, S, many,
           [&](int m, float2, int i2, int i1) {
@@ -433,11 +435,12 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
     return false;
   const int nmore = *S.cnt();
   const int rw = S.L.rw, cells = rw * S.L.rh;
-  auto fetch = [&](int k) {
+  const bool split = shares > 1;
+  auto fetch = [&](int k, int buf) {
     const float* inv = A.sw + (int64_t)k * A.mcap;
     const float* fk = A.a.dev + (int64_t)k * A.mcap;
-    float2* kv = S.kv() + (k & 1) * n2;
-    float2* mkv = S.mkv() + (k & 1) * kGridMore;
+    float2* kv = S.kv() + buf * n2;
+    float2* mkv = S.mkv() + buf * kGridMore;
     for (int ci = threadIdx.x; ci < cells; ci += blockDim.x) {
       const int ry = ci / rw, i2 = ry * s2 + ci - ry * rw, m = S.gi()[i2];
       if (m >= 0) {
@@ -458,12 +461,13 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
     const float2 pp = has ? make_float2(A.b.off[j], A.b.off[A.ccap + j]) : make_float2(0.f, 0.f);
     uint32_t empty = 0;
     DF F[Q];
-    fetch(0);
+    int buf = 0;
+    fetch(blockIdx.y, 0);
 #pragma unroll 1
-    for (int k = 0; k < Q; ++k) {
+    for (int k = blockIdx.y; k < Q; k += shares, buf ^= 1) {
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
-      if (k + 1 < Q) fetch(k + 1);
+      if (k + shares < Q) fetch(k + shares, buf ^ 1);
       if (!has) continue;
       const float cdx = A.L.cdf[k][0], cdy = A.L.cdf[k][1];
       const float bxr = pp.x - cdx, byr = pp.y - cdy;
@@ -478,7 +482,7 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
       };
       const int i0 = (by + loy) * s2 + bx + lox;
       const float2* o0 = S.xy() + i0;
-      const float2* kv0 = S.kv() + (k & 1) * n2 + i0;
+      const float2* kv0 = S.kv() + buf * n2 + i0;
       const float* r0 = S.fl() + (by + loy) * s1 + bx + lox;
       if (nx <= W && ny <= W) {
         float cx[W];
@@ -499,13 +503,21 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
       }
       if (nmore)
         window_more(S, by + loy, ny, bx + lox, nx, [&](int q, int r, int c) {
-          one(S.mxy()[q], S.mfl()[q], S.mkv()[(k & 1) * kGridMore + q], canon_c<float>(c - bx, cdx, pp.x),
+          one(S.mxy()[q], S.mfl()[q], S.mkv()[buf * kGridMore + q], canon_c<float>(c - bx, cdx, pp.x),
               canon_c<float>(r - by, cdy, pp.y));
         });
-      F[k] = gather_total(A.L.wf[k], A.L.wlo[k], s.hi, s.lo, s.sb);
-      if (F[k].hi < A.eps) empty |= 1u << k;
+      const DF Fk = gather_total(A.L.wf[k], A.L.wlo[k], s.hi, s.lo, s.sb);
+      if (Fk.hi < A.eps) empty |= 1u << k;
+      if (split) {
+        A.cpfhi[(int64_t)k * A.ccap + j] = Fk.hi;
+        A.cpflo[(int64_t)k * A.ccap + j] = Fk.lo;
+      } else {
+        F[k] = Fk;
+      }
     }
-    if (has) {
+    if (split) {
+      if (has && empty) atomicOr(A.emask + j, empty);
+    } else if (has) {
       A.emask[j] = empty;
       if (fuse && !empty) {
         emit_full<Q>(A, j, F);
@@ -523,6 +535,18 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
 }
 
 // ---- kernels ----------------------------------------------------------------------------------------
+//
+// Weights and gather of few moments: up to gridDim.y blocks share a tile's directions (k = blockIdx.y,
+// blockIdx.y + shares, ...), since one block per SM waits on its own loads and sums.  Shares (direction_shares): as many as the
+// blocks of the moments' tiles (256 cells, one moment each where the store is full) still run at once, and
+// the directions in equal parts.  The gather then leaves its sums to the emit pass.  D2Q7 at R = 4
+// cells, 5 k to 30 k moments in 24 k to 63 k cells: weights 93 -> 33 us, gather 167 -> 47.  Every block of a tile
+// stages the same items and finds the same fault, and the first defers it.
+// This launch's shares (the moments the step began with); slots 0: one.
+template <int Q>
+__device__ __forceinline__ int grid_shares(const Args<Q, 2, PF32>& A) {
+  return A.share_slots ? min(direction_shares<Q>(*A.a.count, A.share_slots), (int)gridDim.y) : 1;
+}
 
 template <int Q, int W>
 __global__ void __launch_bounds__(256, 4) k_thin_refine_grid(const __grid_constant__ Args<Q, 2, PF32> A,
@@ -542,10 +566,12 @@ __global__ void __launch_bounds__(256, 4) k_weights_grid(const __grid_constant__
                                                         const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
                                                         int* fb_tiles, int* fb_count) {
   extern __shared__ __align__(16) unsigned char smem[];
+  const int shares = grid_shares<Q>(A);
+  if ((int)blockIdx.y >= shares) return;
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
-    if (!weights_grid_tile<Q, W>(A, T, I, G, smem)) defer_tile(tb, fb_tiles, fb_count);
+    if (!weights_grid_tile<Q, W>(A, T, I, G, shares, smem) && blockIdx.y == 0) defer_tile(tb, fb_tiles, fb_count);
     __syncthreads();
   }
 }
@@ -555,11 +581,14 @@ __global__ void __launch_bounds__(256, 4) k_gather_grid(const __grid_constant__ 
                                                        const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
                                                        int* fb_tiles, int* fb_count, int fuse) {
   extern __shared__ __align__(16) unsigned char smem[];
+  const int shares = grid_shares<Q>(A);
+  if ((int)blockIdx.y >= shares) return;
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
     // a negative density or an f that is not finite anywhere (noted by the collision): no grid tile
-    if (*A.odd_f || !gather_grid_tile<Q, W>(A, T, I, G, fuse != 0, smem)) defer_tile(tb, fb_tiles, fb_count);
+    if ((*A.odd_f || !gather_grid_tile<Q, W>(A, T, I, G, shares, fuse != 0, smem)) && blockIdx.y == 0)
+      defer_tile(tb, fb_tiles, fb_count);
     __syncthreads();
   }
 }
