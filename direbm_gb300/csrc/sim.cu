@@ -1013,26 +1013,26 @@ __global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D,
         hi[a] = (int)floor(p[a] + A.R + A.tiny);
       }
       CSum sws[Q];
+      // window rows as runs of consecutive cells, whose items are consecutive; few points have gaps, so
+      // this waits on its loads: a cell at a time took 31 us at R = 4 cells where this takes 17
 #pragma unroll 1
       for (int gz = lo[2]; gz <= hi[2]; ++gz)
 #pragma unroll 1
-        for (int gy = lo[1]; gy <= hi[1]; ++gy)
-#pragma unroll 1
-          for (int gx = lo[0]; gx <= hi[0]; ++gx) {
-            const int dS[3] = {gx, gy, gz};
-            real cc[3] = {0, 0, 0};
-#pragma unroll
-            for (int a = 0; a < D; ++a) cc[a] = canon_c<real>(dS[a], (real)0, p[a]);
-            if (cell_d2_lower<D, real>(cc) > A.R2) continue;
-            uint32_t Hg;
-            if (!cell_at<D>(I, Gc[0] + gx, Gc[1] + gy, Gc[2] + gz, &Hg)) continue;
-            const uint32_t c0 = A.b.start[Hg], c1 = A.b.start[Hg + 1];
-            for (uint32_t c = c0; c < c1; ++c) {
+        for (int gy = lo[1]; gy <= hi[1]; ++gy) {
+          row_runs<D>(I, Gc[0], Gc[1] + gy, Gc[2] + gz, lo[0], hi[0], [&](uint32_t g0, uint32_t g1, int shift) {
+            const int x0 = (int)((g0 - I.base) % (uint32_t)I.dims[0]) + shift - Gc[0];  // window column of g0
+            const uint32_t c1 = A.b.start[g1 + 1];
+#pragma unroll 4
+            for (uint32_t c = A.b.start[g0]; c < c1; ++c) {
               const uint32_t both = A.emask[c] & em;
               if (!both) continue;
-              real o[3] = {0, 0, 0}, e[3];
+              const int dS[3] = {x0 + (int)(A.b.cell[c] - g0), gy, gz};
+              real cc[3] = {0, 0, 0}, o[3] = {0, 0, 0}, e[3];
 #pragma unroll
-              for (int a = 0; a < D; ++a) o[a] = A.b.off[(int64_t)a * A.ccap + c];
+              for (int a = 0; a < D; ++a) {
+                cc[a] = canon_c<real>(dS[a], (real)0, p[a]);
+                o[a] = A.b.off[(int64_t)a * A.ccap + c];
+              }
               const real d2 = canon_d2<D, real>(o, cc, e);
               if (d2 <= A.R2) {
                 const real w = A.R - rn_sqrt(d2);
@@ -1044,7 +1044,8 @@ __global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D,
                 }
               }
             }
-          }
+          });
+        }
       if constexpr (!std::is_same<P, PF64>::value) {
 #pragma unroll
         for (int k = 0; k < Q; ++k) swf[k] = sws[k].value();

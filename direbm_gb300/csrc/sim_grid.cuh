@@ -537,8 +537,8 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
 // ---- kernels ----------------------------------------------------------------------------------------
 //
 // Weights and gather of few moments: up to gridDim.y blocks share a tile's directions (k = blockIdx.y,
-// blockIdx.y + shares, ...), since one block per SM waits on its own loads and sums.  Shares (direction_shares): as many as the
-// blocks of the moments' tiles (256 cells, one moment each where the store is full) still run at once, and
+// blockIdx.y + shares, ...), since one block per SM waits on its own loads and sums.  Shares
+// (direction_shares): as many as the blocks of the moments' tiles (256 cells, one moment each where the store is full) still run at once, and
 // the directions in equal parts.  The gather then leaves its sums to the emit pass.  D2Q7 at R = 4
 // cells, 5 k to 30 k moments in 24 k to 63 k cells: weights 93 -> 33 us, gather 167 -> 47.  Every block of a tile
 // stages the same items and finds the same fault, and the first defers it.
