@@ -224,11 +224,13 @@ struct Arena {
   template <class T>
   int get(T** p, int64_t count) {
     if (!base) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      DBM_CUDA(cudaStreamIsCapturing(s, &cap));
       cudaMemPool_t pool = nullptr;
-      DBM_TRY(stage_pool(&pool));
+      if (cap == cudaStreamCaptureStatusNone) DBM_TRY(stage_pool(&pool));  // a captured graph owns its memory
       void* q = nullptr;
-      const cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, pool, s);
-      if (e != cudaSuccess) { set_last_error("cudaMallocFromPoolAsync: %s", cudaGetErrorString(e)); return DBM_ERR_CUDA; }
+      const cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, bytes, pool, s) : cudaMallocAsync(&q, bytes, s);
+      if (e != cudaSuccess) { set_last_error("stage temporaries: %s", cudaGetErrorString(e)); return DBM_ERR_CUDA; }
       base = (char*)q;
     }
     const size_t sz = ((size_t)std::max<int64_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
