@@ -57,10 +57,11 @@ KERNEL_BYTES = {
     "thin_refine": ("moment+cell", 4 * (1 + Q9) + 4 + 4 * D2, 4 + 16),
     # per component: read offsets (8) + cell (4) once per moment, write sw (4); CP reads (12/CP)
     "weights": ("moment+cp", 4 * D2 + 4 + 4 * Q9, 12),
-    # per moment: offsets + rho + dev + sw (8+4+36+36) + starts; per CP: cell+offsets (12) + cpf (72) + mask (4)
-    "gather": ("moment+cp", 4 * D2 + 4 * (1 + Q9) + 4 * Q9 + 4, 12 + 8 * Q9 + 4),
-    # per CP: read cpf (72) + mask (4) + cell/off (12); write rho + dev (40)
-    "emit": ("cp", 0, 8 * Q9 + 4 + 12 + 4 * (1 + Q9)),
+    # per moment: offsets + rho + dev + sw (8+4+36+36) + starts; per CP: cell+offsets (12), write rho + dev
+    # (40) + mask (4): the gather emits the points without an empty direction
+    "gather": ("moment+cp", 4 * D2 + 4 * (1 + Q9) + 4 * Q9 + 4, 12 + 4 * (1 + Q9) + 4),
+    # per CP: read mask (4); points with empty directions are few
+    "emit": ("cp", 0, 4),
     # per moment: read rho + dev, write dev
     "collide": ("moment", 4 * (1 + Q9) + 4 + 4 * Q9, 0),
     # per CP, radix path: 3 passes x (hist read 4 + scatter read 8 + write 8) + compaction (8) +
@@ -70,9 +71,9 @@ KERNEL_BYTES = {
 
 # DRAM bytes per input moment measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum) for
 # one launch of k_gather_ds (the dense-stencil gather this workload runs) on a 4.18 M-moment case
-# of this workload (its first 64 members, 16x16 tiles): 419.6 MB read + 267.4 MB written.  Traffic
+# of this workload (its first 64 members, 16x16 tiles): 423.8 MB read + 163.1 MB written.  Traffic
 # grows with the moments, so a full launch's traffic is this times M.
-KERNEL_TRAFFIC_PER_MOMENT = {"gather": 164.2}
+KERNEL_TRAFFIC_PER_MOMENT = {"gather": 140.3}
 
 # Per point-step byte model of the method (components materialised as 12-byte sort records):
 # B = M(Qs+b_p) + Nc k_b + 2 Nc k_b + 3(Nc k_b + M(Qs+b_p)) + 3 P b_p + P(Qs+b_p), with P ~ M,

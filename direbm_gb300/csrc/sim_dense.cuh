@@ -32,7 +32,7 @@
 // weights 78 %, gather 70 %; DRAM 5-10 %).  Ensemble of 15.5 M moments, 16 x 16 tiles, ms per step,
 // branching 4 x 4 stencil before / now: thin + refine 2.33 / 1.70, weights 2.92 / 1.66, gather with
 // emit 4.51 / 3.50; whole step 10.2 / 7.3, and 11.3 / 9.7 after 100 steps (two-item cells).  One
-// 64 x 64 box, whole step: 140 us / 64 us.
+// 64 x 64 box, whole step: 140 us / 60 us.
 #pragma once
 
 #include "sim_tiled.cuh"

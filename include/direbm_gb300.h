@@ -87,18 +87,20 @@ int dbm_disperse_f32(const float* d_pos_m, const float* d_f_m, int64_t m, int la
 /* create_control_points: direbm/warp/propagation.py:39-68,130-153.  Cell key (floor(x/cs),
  * floor(y/cs)), stable radix sort, run-length encode, exclusive scan, sequential FP32 centroid
  * per run in sorted order.  d_cp_pos needs room for nc points; *p_out receives P (this call
- * synchronises the stream, as the reference's run_count.numpy() did). */
+ * synchronises the stream, as the reference's run_count.numpy() did).
+ * The three functions below read the points' bounds back first, one short host wait each, to index them
+ * with short keys; refine and resample leave that out while their stream is being captured.  Their
+ * temporaries come from a stream-ordered pool of the device that keeps up to 64 MB. */
 int dbm_create_control_points_f32(const float* d_pos_c, int64_t nc, float cs, float* d_cp_pos,
                                   int64_t* p_out, void* stream);
 /* refine_control_points: direbm/warp/propagation.py:77-112,249-275. */
 int dbm_refine_control_points_f32(const float* d_cp_pos, int64_t p, const float* d_pos_c, const float* d_val_c,
                                   const int32_t* d_dir_c, int64_t nc, float dx, int kappa_hard,
                                   float* d_new_pos, void* stream);
-/* resample: direbm/warp/propagation.py:156-246 (scatter + gap fill + emit).  The scatter keeps the
- * reference's form -- each component sends (dx - d)/sw * f to every control point within dx --
- * with its float atomics (propagation.py:186) replaced by pair records, a stable sort by (control
- * point, direction) and dbm_segmented_sum_f32, so the result is deterministic.  Synchronises the
- * stream once (the record count sizes the sort).  out_f is (P, Q). */
+/* resample: direbm/warp/propagation.py:156-246 (scatter + gap fill + emit).  The reference's scatter with
+ * float atomics (propagation.py:186) -- each component sends (dx - d)/sw * f to every control point within
+ * dx -- is a gather here: every control point sums its components in a fixed order, so the result is
+ * deterministic.  Components with a direction outside [0, Q) are dropped.  out_f is (P, Q). */
 int dbm_resample_f32(const float* d_pos_c, const float* d_val_c, const int32_t* d_dir_c, int64_t nc,
                      const float* d_cp_pos, int64_t p, float dx, const float* d_f_rest, int lattice,
                      float eps, float* d_out_pos, float* d_out_f, void* stream);
@@ -217,7 +219,8 @@ int dbm_sim_use_graphs(dbm_sim* sim, int32_t on);
  * r (none when that sum is below 1e-8).  Needs a moment capacity of 2 x cells (DBM_ERR_CAPACITY
  * otherwise); runs on the untiled kernels; the tape (dbm_tape_*) refuses a simulator with it on. */
 #define DBM_OPT_KAPPA_SOFT 5
-/* DBM_OPT_BRICK_WIDTH: the untiled window kernels (3D, obstacles, the soft spawn, tiles off) give
+/* DBM_OPT_BRICK_WIDTH: the untiled window kernels (FP64, near obstacles, 3D radii without a grid kernel,
+ * the soft spawn, tiles off) give
  * each block a brick of 256 cells, this many along x (a power of two, 4..32 in 3D, 8..64 in 2D;
  * default 8 in 3D, 16 in 2D); results do not depend on it.  direbm_gb300.autotune picks it. */
 #define DBM_OPT_BRICK_WIDTH 6
@@ -226,7 +229,8 @@ int dbm_sim_use_graphs(dbm_sim* sim, int32_t on);
  * window rows per reference point and shift it for each direction instead of building a window
  * per (point, direction) (default 1).  Results are bit-identical either way. */
 #define DBM_OPT_SHIFTED_WINDOWS 7
-/* DBM_OPT_DENSE_STENCIL (2D, FP32 store, with the shifted windows): a tile whose cells each hold at
+/* DBM_OPT_DENSE_STENCIL (FP32 store; also the grid windows of displacements that are not whole cells, of
+ * R near 4 cells and of 3D): a tile whose cells each hold at
  * most two moments and two control points (in D2Q9 runs with dx = cell, almost every cell holds
  * exactly one) is staged as a dense grid -- second items in a per-tile list of 32 -- and every
  * window becomes a fixed 4 x 4 block of cells; other tiles take the row-segment loops in a second
