@@ -34,6 +34,9 @@ template <int Q, int D, class P>
 __global__ void __launch_bounds__(256) k_collide(const __grid_constant__ Args<Q, D, P> A) {
   using real = typename P::real;
   const uint32_t M = *A.a.count;
+  if (A.clear_start)  // the counts of k_place_count; a clear of its own is a launch of 2 us
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= A.ncells; c += gridDim.x * blockDim.x)
+      A.b.start[c] = 0u;
   for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
     const uint32_t g = A.a.cell[m];
     const int b = find_instance(A.inst_base, A.n_inst, g);
@@ -616,6 +619,7 @@ __global__ void __launch_bounds__(256) k_place(const __grid_constant__ Args<Q, D
     keys[j] = G;
     vals[j] = F;
     A.b.cell[j] = G;
+    if (A.clear_emask) A.emask[j] = 0u;
 #pragma unroll
     for (int a = 0; a < D; ++a) A.b.off[(int64_t)a * A.ccap + j] = A.foff[(int64_t)a * A.ncells + F];
   }
@@ -2223,6 +2227,20 @@ struct SimImpl : SimBase {
     int* const fb = brick3_path() ? d_fb3 : d_fb;
     A.odd_f = fb ? fb + 3 : nullptr;
     if (fb) DBM_CUDA(cudaMemsetAsync(fb, 0, 4 * sizeof(int), s));
+    // the gather's empty masks: written whole by one block per tile, else combined from zero
+    bool dense = false, split = false, shared = false;  // shared: split if the device says so
+    if constexpr (kTiles) {
+      if (tiled_path() && shift_ok && use_shift && use_dense) {
+        dense = true;
+        split = split_ds[2] > 1;
+      } else if (grid_path()) {
+        dense = true;
+        shared = grid_y > 1;
+      }
+    }
+    const bool from_zero = !dense || split || shared;
+    A.clear_start = place_path() ? 1 : 0;
+    A.clear_emask = place_path() && from_zero ? 1 : 0;
     k_collide<Q, D, P><<<gm, 256, 0, s>>>(A);
     DBM_LAUNCH_CHECK();
     if (untiled) {
@@ -2274,7 +2292,6 @@ struct SimImpl : SimBase {
     if (place_path()) {
       // counts per final cell -> cell starts (and P) by one scan -> each point's slot
       const unsigned gf = std::min<unsigned>(div_up(ncells, 256), (unsigned)sm_count() * 16);
-      DBM_CUDA(cudaMemsetAsync(A.b.start, 0, ((size_t)ncells + 1) * 4, s));
       k_place_count<Q, D, P><<<gf, 256, 0, s>>>(A, A.b.start);
       DBM_LAUNCH_CHECK();
       DBM_TRY(scan_exclusive_u32(A.b.start, A.b.start, (int64_t)ncells + 1, nullptr, A.d_P, place_tmp, s));
@@ -2349,18 +2366,8 @@ struct SimImpl : SimBase {
     if (upto <= 4) return DBM_OK;
     // the dense gather writes every control point's empty mask and, unless the step keeps its
     // intermediates, emits the points without an empty direction itself
-    bool dense = false, split = false, shared = false;  // shared: split if the device says so
-    if constexpr (kTiles) {
-      if (tiled_path() && shift_ok && use_shift && use_dense) {
-        dense = true;
-        split = split_ds[2] > 1;
-      } else if (grid_path()) {
-        dense = true;
-        shared = grid_y > 1;
-      }
-    }
     const int fuse = ((dense && !split) || brick3_path()) && !A.write_trace ? 1 : 0;
-    if (!dense || split || shared) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
+    if (from_zero && !A.clear_emask) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (kTiles) {
       if (tiled_path()) {
         bool shifted = false;
