@@ -20,6 +20,8 @@ from .sim import _require_cuda, _stream
 
 def _edges(edges, dev):
     """The axes' edge arrays on the device, in one copy that the host does not wait for."""
+    if torch.cuda.is_current_stream_capturing():  # a replay would read host memory that is reused by then
+        raise RuntimeError("bin_fields: the edges are host data; the call cannot be captured in a graph")
     sizes = [len(e) for e in edges]
     host = torch.empty(sum(sizes), dtype=torch.float64, pin_memory=True)
     np.concatenate([np.asarray(e, np.float64) for e in edges], out=host.numpy())

@@ -64,3 +64,20 @@ def test_bin_fields_bits(kind, lattice):
     out = run(x, f, *edges, lattice)
     for v in range(1 + D):
         np.testing.assert_array_equal(out[v].cpu().numpy(), ref[v])
+
+
+def test_capture_is_refused():
+    import torch
+    from direbm_gb300.fields import bin_fields_device
+    from direbm_gb300.lattices import get
+
+    lat = get("D2Q9")
+    x = torch.zeros((4, 2), dtype=torch.float64, device="cuda")
+    f = torch.ones((4, lat.Q), dtype=torch.float64, device="cuda")
+    edges = np.array([-1.0, 0.5, 1.0])
+    mass, _, _ = bin_fields_device(x, f, edges, edges, lat)
+    with pytest.raises(RuntimeError, match="captured"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            bin_fields_device(x, f, edges, edges, lat)
+    again, _, _ = bin_fields_device(x, f, edges, edges, lat)
+    assert torch.equal(mass, again) and float(mass[0, 0]) == 4.0 * lat.Q
