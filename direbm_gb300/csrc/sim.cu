@@ -34,7 +34,9 @@ template <int Q, int D, class P>
 __global__ void __launch_bounds__(256) k_collide(const __grid_constant__ Args<Q, D, P> A) {
   using real = typename P::real;
   const uint32_t M = *A.a.count;
-  if (A.clear_start)  // the counts of k_place_count; a clear of its own is a launch of 2 us
+  // The counts of k_place_count; a clear of its own is a launch of 2 us.  Ten steps of 64 x 64 cells: 620 us
+  // with clears of these and of the empty masks (k_place), 601 without.
+  if (A.clear_start)
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= A.ncells; c += gridDim.x * blockDim.x)
       A.b.start[c] = 0u;
   for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
