@@ -1668,15 +1668,18 @@ struct SimImpl : SimBase {
   }
 
   // The 3D grid kernels serve windows of ceil(2 R) + 1 = 4 cells (1 < R <= 1.5, the radii in use) whose
-  // region lies within kHalo3 cells of a brick.
+  // region lies within kHalo3 cells of a brick: the exact ranges, and the four cells from a window's first
+  // one, which the kernels read also where the exact range holds three (a displacement longer than R).
   int init_brick3(const LatHost& LH, double R) {
     if constexpr (D == 3 && std::is_same<P, PF32>::value) {
       if ((int)std::ceil(2 * R - 1e-3) + 1 != 4) return DBM_OK;
-      const double tiny = 2e-4;
+      const double tiny = 2e-4;  // beyond the kernels' margin; half of theirs where that draws a window in
       for (int k = 0; k < Q; ++k)
         for (int a = 0; a < 3; ++a) {
           const double cd = std::fabs(LH.c[k][a] * desc.dx / desc.cell) * (1 + 1e-6);
-          if (std::floor(-cd - R - tiny) < -kHalo3 || std::floor(1 + cd + R + tiny) > kHalo3) return DBM_OK;
+          if (std::floor(-cd - R - tiny) < -kHalo3 || std::floor(1 + cd + R + tiny) > kHalo3 ||
+              std::floor(1 + cd - R - 0.5 * (double)args.tiny) + 3 > kHalo3)
+            return DBM_OK;
         }
       const void* k3[3] = {(const void*)k_brick3<Q, 0>, (const void*)k_brick3<Q, 1>, (const void*)k_brick3<Q, 2>};
       for (int i = 0; i < 3; ++i)

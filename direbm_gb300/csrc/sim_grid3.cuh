@@ -30,7 +30,9 @@ namespace dbm {
 
 constexpr int kBrick3 = 8;  // cells per side of a brick
 constexpr int kThreads3 = kBrick3 * kBrick3 * kBrick3;
-constexpr int kHalo3 = 3;   // cells of halo on each side: 1 < R <= 1.5 and displacements of at most one cell
+// Cells of halo on each side: 1 < R <= 1.5 and displacements that keep every window, and the four cells from
+// its first one, inside (the host checks; up to R where that is 1.5, so one cell in use).
+constexpr int kHalo3 = 3;
 constexpr int kW3 = kBrick3 + 2 * kHalo3;
 constexpr int kCells3 = kW3 * kW3 * kW3;
 // Row and plane strides of the records: eight lanes of a row read one 128-byte line of 16-byte records,
