@@ -1467,7 +1467,6 @@ struct SimImpl : SimBase {
   // 3D grid kernels (k_brick3): bricks of 8^3 cells away from obstacles, the other bricks (8 x 8 x 4, for
   // the untiled kernels), and per stage the bricks they defer (d_fb3[0..2] counts, [3] odd_f, + 4 list)
   bool brick3_ok = false;
-  bool bricks3_stale = true;
   Brick *d_bricks3 = nullptr, *d_near3 = nullptr;
   int nbricks3 = 0, nnear3 = 0;
   int* d_fb3 = nullptr;
@@ -1685,15 +1684,18 @@ struct SimImpl : SimBase {
       for (int i = 0; i < 3; ++i)
         DBM_CUDA(cudaFuncSetAttribute(k3[i], cudaFuncAttributeMaxDynamicSharedMemorySize, grid3_layout(i).total));
       brick3_ok = true;
+      DBM_TRY(make_bricks3());
     }
     return DBM_OK;
   }
 
   // The brick lists of the 3D grid kernels: a brick belongs to the untiled kernels when a point of it
   // could meet a bounced component, or a moment of its region be one (the obstacle's reach, set_obstacle).
+  // Made at creation and when an obstacle changes, in buffers for all bricks in either list: a step, or a
+  // new inflow velocity, allocates and waits for nothing.
   int make_bricks3() {
     if constexpr (D == 3 && std::is_same<P, PF32>::value) {
-      if (!brick3_ok || !bricks3_stale) return DBM_OK;
+      if (!brick3_ok) return DBM_OK;
       std::vector<Brick> far, near;
       for (int i = 0; i < (int)inst_h.size(); ++i) {
         const InstK& I = inst_h[i];
@@ -1719,21 +1721,17 @@ struct SimImpl : SimBase {
               }
             }
       }
-      DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the old lists
-      release(d_bricks3);
-      release(d_near3);
-      release(d_fb3);
-      d_bricks3 = d_near3 = nullptr;
-      d_fb3 = nullptr;
-      DBM_TRY(alloc(&d_bricks3, (int64_t)far.size()));
-      DBM_TRY(alloc(&d_near3, (int64_t)near.size()));
-      DBM_TRY(alloc(&d_fb3, (int64_t)far.size() + 4));
+      if (!d_bricks3) {  // at creation, with every brick clear
+        DBM_TRY(alloc(&d_bricks3, (int64_t)far.size()));
+        DBM_TRY(alloc(&d_near3, 2 * (int64_t)far.size()));
+        DBM_TRY(alloc(&d_fb3, (int64_t)far.size() + 4));
+      }
+      if (own) DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the old lists
       DBM_CUDA(cudaMemcpy(d_bricks3, far.data(), sizeof(Brick) * far.size(), cudaMemcpyHostToDevice));
       DBM_CUDA(cudaMemcpy(d_near3, near.data(), sizeof(Brick) * near.size(), cudaMemcpyHostToDevice));
+      if (nbricks3 != (int)far.size() || nnear3 != (int)near.size()) invalidate_graphs();  // launches hold the sizes
       nbricks3 = (int)far.size();
       nnear3 = (int)near.size();
-      bricks3_stale = false;
-      invalidate_graphs();  // captured launches hold the lists
     }
     return DBM_OK;
   }
@@ -2422,7 +2420,6 @@ struct SimImpl : SimBase {
 
   int step(int n, cudaStream_t s) override {
     if (n <= 0) return DBM_OK;
-    DBM_TRY(make_bricks3());
     ++version;
     DBM_CUDA(cudaEventRecord(ev_in, s));
     DBM_CUDA(cudaStreamWaitEvent(own, ev_in, 0));
@@ -2458,7 +2455,6 @@ struct SimImpl : SimBase {
   // receives the 6 stage durations (collide, thin+refine, compaction+sort+finalize, weights,
   // gather, emit) measured on the stream the kernels run on.
   int profile_step(float* stage_ms, cudaStream_t s) override {
-    DBM_TRY(make_bricks3());
     ++version;
     cudaEvent_t ev[7];
     for (auto& e : ev) DBM_CUDA(cudaEventCreate(&e));
@@ -2480,7 +2476,6 @@ struct SimImpl : SimBase {
   }
 
   int step_partial(int upto, cudaStream_t s) override {
-    DBM_TRY(make_bricks3());
     trace_on = 1;
     ++version;
     DBM_CUDA(cudaEventRecord(ev_in, s));
@@ -2497,7 +2492,6 @@ struct SimImpl : SimBase {
   // One full step launched stage by stage with every intermediate kept, and `h` called before the
   // collision and after the emit (the adjoint records its tape there).
   int step_hooked(StepHook* h, cudaStream_t s) override {
-    DBM_TRY(make_bricks3());
     const int keep = trace_on;
     ++version;
     trace_on = 1;
@@ -2582,7 +2576,8 @@ struct SimImpl : SimBase {
     } else {
       I.has_obs = 0;
     }
-    return push_instances();
+    DBM_TRY(push_instances());
+    return make_bricks3();
   }
 
   // An inflow layer in instance `b`: moments in the first `width` cell columns (x) are set to the
@@ -2598,7 +2593,6 @@ struct SimImpl : SimBase {
   int push_instances() {
     DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the table
     DBM_CUDA(cudaMemcpy(dinst, inst_h.data(), sizeof(InstK) * inst_h.size(), cudaMemcpyHostToDevice));
-    bricks3_stale = true;
     int any = 0;
     for (auto& I : inst_h) any |= I.has_obs;
     if (any != args.any_obstacle) {
