@@ -473,6 +473,9 @@ __global__ void __launch_bounds__(256) k_cp_fill(const float2* __restrict__ cps,
 
 using namespace dbm;
 
+// Points are indexed in 32 bits, with room for a grid's stride above the last.
+constexpr int64_t kMaxPoints = 1ll << 31;
+
 static int check_2d(int lattice) {
   const LatHost* h = lat_host(lattice);
   if (!h || h->D != 2) {
@@ -541,7 +544,8 @@ int dbm_create_control_points_f32(const float* pos_c, int64_t nc, float cs, floa
 int dbm_refine_control_points_f32(const float* cp, int64_t p, const float* pos_c, const float* val_c,
                                   const int32_t* dir_c, int64_t nc, float dx, int kappa_hard, float* new_pos,
                                   void* stream) {
-  if (p < 0 || nc < 0 || !(dx > 0.f) || (p > 0 && (!cp || !new_pos)) || (nc > 0 && (!pos_c || !val_c || !dir_c))) {
+  if (p < 0 || nc < 0 || nc > kMaxPoints || !(dx > 0.f) || (p > 0 && (!cp || !new_pos)) ||
+      (nc > 0 && (!pos_c || !val_c || !dir_c))) {
     set_last_error("refine_control_points: bad arguments");
     return DBM_ERR_INVALID;
   }
@@ -569,7 +573,8 @@ int dbm_resample_f32(const float* pos_c, const float* val_c, const int32_t* dir_
                      int64_t p, float dx, const float* f_rest, int lattice, float eps, float* out_pos, float* out_f,
                      void* stream) {
   DBM_TRY(check_2d(lattice));
-  if (p < 0 || nc < 0 || !(dx > 0.f) || (p > 0 && (!cp || !out_pos || !out_f || !f_rest)) ||
+  if (p < 0 || nc < 0 || p > kMaxPoints || nc > kMaxPoints || !(dx > 0.f) ||
+      (p > 0 && (!cp || !out_pos || !out_f || !f_rest)) ||
       (nc > 0 && (!pos_c || !val_c || !dir_c))) {
     set_last_error("resample: bad arguments");
     return DBM_ERR_INVALID;
