@@ -118,7 +118,8 @@ struct PointIndex {
 };
 
 // Cells along one axis within 1 + m of the quotient f, m above the rounding of the quotients and of the
-// distance (relative 2^-22), at most two away; from 2^40 on, where floats lie further apart than dx, its own.
+// distance (relative 2^-22), at most two away; from 2^40 on, an infinite quotient included, where floats lie
+// further apart than dx, its own.
 __device__ __forceinline__ void near_cells(float f, long long* lo, long long* hi) {
   const long long c = (long long)floorf(f);
   *lo = *hi = c;
@@ -134,7 +135,7 @@ __device__ __forceinline__ void near_cells(float f, long long* lo, long long* hi
 template <class F>
 __device__ __forceinline__ void near_points(const PointIndex& ix, float x, float y, float dx, F&& body) {
   const float fx = __fdiv_rn(x, dx), fy = __fdiv_rn(y, dx);
-  if (!isfinite(fx) || !isfinite(fy) || ix.n == 0) return;  // at no finite distance from any point
+  if (ix.n == 0) return;
   long long x0, x1, y0, y1;
   near_cells(fx, &x0, &x1);
   near_cells(fy, &y0, &y1);
