@@ -582,6 +582,12 @@ int dbm_resample_f32(const float* pos_c, const float* val_c, const int32_t* dir_
   }
   if (p == 0) return DBM_OK;
   cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  DBM_CUDA(cudaStreamIsCapturing(s, &cap));
+  if (nc > 0 && cap != cudaStreamCaptureStatusNone) {  // as ever: the call waits for the stream
+    set_last_error("resample: the call synchronises and cannot be captured");
+    return DBM_ERR_STATE;
+  }
   return dispatch_lattice(lattice, [&](auto tag) -> int {
     using LT = decltype(tag);
     if constexpr (LT::D == 2) {

@@ -89,7 +89,7 @@ int dbm_disperse_f32(const float* d_pos_m, const float* d_f_m, int64_t m, int la
  * per run in sorted order.  d_cp_pos needs room for nc points; *p_out receives P (this call
  * synchronises the stream, as the reference's run_count.numpy() did).
  * The three functions below read the points' bounds back first, one short host wait each, to index them
- * with short keys; refine and resample leave that out while their stream is being captured.  Their
+ * with short keys; the refine leaves that out while its stream is being captured.  Their
  * temporaries come from a stream-ordered pool of the device that keeps up to 64 MB. */
 int dbm_create_control_points_f32(const float* d_pos_c, int64_t nc, float cs, float* d_cp_pos,
                                   int64_t* p_out, void* stream);
@@ -100,7 +100,8 @@ int dbm_refine_control_points_f32(const float* d_cp_pos, int64_t p, const float*
 /* resample: direbm/warp/propagation.py:156-246 (scatter + gap fill + emit).  The reference's scatter with
  * float atomics (propagation.py:186) -- each component sends (dx - d)/sw * f to every control point within
  * dx -- is a gather here: every control point sums its components in a fixed order, so the result is
- * deterministic.  Components with a direction outside [0, Q) are dropped.  out_f is (P, Q). */
+ * deterministic.  Components with a direction outside [0, Q) are dropped.  out_f is (P, Q).  Synchronises,
+ * so a captured stream is refused (DBM_ERR_STATE; not without components, where there is nothing to read). */
 int dbm_resample_f32(const float* d_pos_c, const float* d_val_c, const int32_t* d_dir_c, int64_t nc,
                      const float* d_cp_pos, int64_t p, float dx, const float* d_f_rest, int lattice,
                      float eps, float* d_out_pos, float* d_out_f, void* stream);
