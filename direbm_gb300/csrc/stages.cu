@@ -7,6 +7,7 @@
 // the cell keys are as short as the points allow (16 bits in place of 64 for 192 x 192 cells, two radix
 // passes in place of eight) and, where the box is not mostly empty, a table of cell starts takes the place
 // of binary searches.  The cells of one x column that a query needs are consecutive: one run of items.
+// The refine alone waits for nothing: its index is a hashed table (HashIndex).
 //
 // The radius test is |a - b| with round-to-nearest FP32 steps and no fused multiply-add, so the
 // pairs found are the oracle's (oracle/stages.py) bit for bit.  Sums run in a fixed order per
@@ -335,10 +336,10 @@ static int build_index(const PointSet& p, const uint32_t (&bounds)[4], bool know
 
 // Components in index order: position, value (expf of it for the refine), direction or weight sum.
 __global__ void k_pack_comps(const float* __restrict__ pos_c, const float* __restrict__ val_c,
-                             const int32_t* __restrict__ dir_c, PointIndex ix, int as_weight,
-                             float4* __restrict__ items) {
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < ix.n; j += gridDim.x * blockDim.x) {
-    const uint32_t c = ix.order[j];
+                             const int32_t* __restrict__ dir_c, const uint32_t* __restrict__ order, uint32_t n,
+                             int as_weight, float4* __restrict__ items) {
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const uint32_t c = order[j];
     const float2 q = load2(pos_c, c);
     const float v = val_c[c];
     items[j] = make_float4(q.x, q.y, as_weight ? expf(v) : v, __int_as_float(dir_c[c]));
@@ -349,21 +350,127 @@ __global__ void k_pack_points(const float* __restrict__ pos, PointIndex ix, floa
     items[j] = load2(pos, ix.order[j]);
 }
 
-// 205 k points, 258 k components: 200 -> 40 us (a search per cell took 16 dependent loads, 25 times).
-__global__ void k_refine(const float* __restrict__ cp, int64_t p, const float4* __restrict__ items, PointIndex ix,
+// The refine's index, which needs no look at the bounds and so leaves the call asynchronous: a table of
+// buckets, one per four components or so, bucket = S column + row modulo its size 2^bits with S near 0.618 of
+// it, so that the rows which a query needs of one column are consecutive and those of the at most five columns
+// lie apart (1 to 4 times S is at least 0.13 of the table from 0; a query has at most five rows): no component
+// is met twice, and the distance sorts out those of other cells.  Blocks of 2^16 columns and rows are displaced
+// against each other, for points whose cells are multiples of a large power of two; a query across a border
+// of blocks (away from the origin, where boxes begin) takes a component only in its own cell's turn.
+struct HashIndex {
+  int bits = 0;
+  uint32_t n = 0;
+  uint32_t* order = nullptr;  // component of each place, by bucket, then in input order
+  uint32_t* start = nullptr;  // first place of each bucket [2^bits + 1]
+
+  __host__ __device__ __forceinline__ uint32_t mask() const { return (1u << bits) - 1u; }
+  __device__ __forceinline__ uint32_t bucket(uint32_t wx, uint32_t wy) const {
+    const uint32_t S = (0x9E3779B9u >> (32 - bits)) | 1u;
+    return (wx * S + wy + block(wx) * 0x85EBCA6Bu + block(wy) * 0xC2B2AE35u) & mask();
+  }
+  static __device__ __forceinline__ uint32_t block(uint32_t w) { return (w + 0x4DB7u) >> 16; }
+};
+
+__global__ void k_hash_keys(const float* __restrict__ pos, HashIndex ix, float cs, uint32_t* __restrict__ keys) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ix.n; i += gridDim.x * blockDim.x) {
+    const float2 q = load2(pos, i);
+    keys[i] = ix.bucket(cell_word(cell_of(q.x, cs)), cell_word(cell_of(q.y, cs)));
+    ix.order[i] = i;
+  }
+}
+__global__ void k_hash_starts(const uint32_t* __restrict__ keys, HashIndex ix) {
+  const uint32_t nb = ix.mask() + 1u;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= nb; c += gridDim.x * blockDim.x) {
+    uint32_t lo = 0, hi = ix.n;
+    while (lo < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1);
+      if (keys[mid] < c) lo = mid + 1; else hi = mid;
+    }
+    ix.start[c] = lo;
+  }
+}
+
+static int hash_bits(int64_t n) {
+  int b = 8;
+  while (b < 31 && (4ll << b) < n) ++b;
+  return b;
+}
+static size_t hash_bytes(int64_t n) {
+  const size_t m = (size_t)std::max<int64_t>(n, 1);
+  return m * (4 * 4 + 16) + radix_tmp_bytes(n) + (((size_t)1 << hash_bits(n)) + 1) * 4 + 8 * 256;
+}
+static int build_hash(const float* pos, int64_t n, float cs, Arena& ar, HashIndex* ix) {
+  cudaStream_t s = ar.s;
+  uint32_t *keys, *k_alt, *v_alt;
+  char* rtmp;
+  ix->n = (uint32_t)n;
+  ix->bits = hash_bits(n);
+  DBM_TRY(ar.get(&keys, n));
+  DBM_TRY(ar.get(&ix->order, n));
+  DBM_TRY(ar.get(&k_alt, n));
+  DBM_TRY(ar.get(&v_alt, n));
+  DBM_TRY(ar.get(&rtmp, (int64_t)radix_tmp_bytes(n)));
+  DBM_TRY(ar.get(&ix->start, (1ll << ix->bits) + 1));
+  k_hash_keys<<<grid_for(n), 256, 0, s>>>(pos, *ix, cs, keys);
+  DBM_LAUNCH_CHECK();
+  bool alt = false;
+  DBM_TRY(radix_sort_pairs<uint32_t>(keys, ix->order, k_alt, v_alt, n, nullptr, ix->bits, rtmp, s, &alt));
+  if (alt) {
+    keys = k_alt;
+    ix->order = v_alt;
+  }
+  k_hash_starts<<<grid_for((1ll << ix->bits) + 1), 256, 0, s>>>(keys, *ix);
+  DBM_LAUNCH_CHECK();
+  return DBM_OK;
+}
+
+// body(it) for the components within dx of p, columns ascending, then rows, then in input order.
+template <class F>
+__device__ __forceinline__ void hash_hits(const HashIndex& ix, const float4* __restrict__ items, float2 p, float dx,
+                                          F&& body) {
+  if (ix.n == 0) return;
+  long long x0, x1, y0, y1;
+  near_cells(__fdiv_rn(p.x, dx), &x0, &x1);
+  near_cells(__fdiv_rn(p.y, dx), &y0, &y1);
+  const uint32_t wx0 = cell_word(x0), wy0 = cell_word(y0), cols = (uint32_t)(x1 - x0), rows = (uint32_t)(y1 - y0);
+  auto within = [&](float4 it) { return dist32(it.x, it.y, p.x, p.y) <= dx; };
+  if (ix.block(wx0) == ix.block(wx0 + cols) && ix.block(wy0) == ix.block(wy0 + rows)) {
+    for (uint32_t c = 0; c <= cols; ++c) {
+      const uint32_t b = ix.bucket(wx0 + c, wy0), b1 = min(b + rows, ix.mask()), over = b + rows - b1;
+      for (uint32_t j = ix.start[b], e = ix.start[b1 + 1u]; j < e; ++j) {
+        const float4 it = items[j];
+        if (within(it)) body(it);
+      }
+      for (uint32_t j = 0, e = ix.start[over]; j < e; ++j) {  // around the table's end
+        const float4 it = items[j];
+        if (within(it)) body(it);
+      }
+    }
+  } else {
+    for (uint32_t c = 0; c <= cols; ++c)
+      for (uint32_t r = 0; r <= rows; ++r) {
+        const uint32_t b = ix.bucket(wx0 + c, wy0 + r);
+        for (uint32_t j = ix.start[b], e = ix.start[b + 1u]; j < e; ++j) {
+          const float4 it = items[j];
+          if (within(it) && cell_word(cell_of(it.x, dx)) == wx0 + c && cell_word(cell_of(it.y, dx)) == wy0 + r) body(it);
+        }
+      }
+  }
+}
+
+// 205 k points, 258 k components: 200 us by searches (16 dependent loads per cell, 25 cells), 40 by either table;
+// the call from 30 k moments (210 k components) 125 us with the read-back of the bounds, 105 without.
+__global__ void k_refine(const float* __restrict__ cp, int64_t p, const float4* __restrict__ items, HashIndex ix,
                          float dx, int kappa_hard, float* __restrict__ out) {
   for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < p; r += (int64_t)gridDim.x * blockDim.x) {
     const float2 q = load2(cp, r);
     uint32_t mask = 0;
     CSum sw, sx, sy;
-    near_points(ix, q.x, q.y, dx, [&](uint32_t j) {
-      const float4 it = items[j];
-      if (dist32(it.x, it.y, q.x, q.y) <= dx) {
-        mask |= 1u << __float_as_int(it.w);
-        sw.add(it.z);
-        sx.add_prod(it.z, it.x);
-        sy.add_prod(it.z, it.y);
-      }
+    hash_hits(ix, items, q, dx, [&](float4 it) {
+      mask |= 1u << __float_as_int(it.w);
+      sw.add(it.z);
+      sx.add_prod(it.z, it.x);
+      sy.add_prod(it.z, it.y);
     });
     if (__popc(mask) <= kappa_hard) {
       store2(out, r, q);
@@ -552,17 +659,13 @@ int dbm_refine_control_points_f32(const float* cp, int64_t p, const float* pos_c
   }
   if (p == 0) return DBM_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  Arena ar(s, index_bytes(nc, true) + 256);
-  PointIndex ix;
+  Arena ar(s, hash_bytes(nc));
+  HashIndex ix;
   float4* items = nullptr;
   if (nc > 0) {
-    const PointSet pts{pos_c, nc, dx};
-    uint32_t bounds[1][4];
-    bool known = false;
-    DBM_TRY(read_bounds(&pts, 1, ar, bounds, &known));
-    DBM_TRY(build_index(pts, bounds[0], known, true, ar, &ix));
+    DBM_TRY(build_hash(pos_c, nc, dx, ar, &ix));
     DBM_TRY(ar.get(&items, nc));
-    k_pack_comps<<<grid_for(nc), 256, 0, s>>>(pos_c, val_c, dir_c, ix, 1, items);
+    k_pack_comps<<<grid_for(nc), 256, 0, s>>>(pos_c, val_c, dir_c, ix.order, ix.n, 1, items);
     DBM_LAUNCH_CHECK();
   }
   k_refine<<<grid_for(p), 256, 0, s>>>(cp, p, items, ix, dx, kappa_hard, new_pos);
@@ -611,7 +714,7 @@ int dbm_resample_f32(const float* pos_c, const float* val_c, const int32_t* dir_
         DBM_TRY(build_index(sets[1], bounds[1], known, true, ar, &ci));
         DBM_TRY(ar.get(&comps, nc));
         DBM_TRY(ar.get(&sw, nc));
-        k_pack_comps<<<grid_for(nc), 256, 0, s>>>(pos_c, val_c, dir_c, ci, 0, comps);
+        k_pack_comps<<<grid_for(nc), 256, 0, s>>>(pos_c, val_c, dir_c, ci.order, ci.n, 0, comps);
         DBM_LAUNCH_CHECK();
         k_comp_sw<<<grid_for(nc), 256, 0, s>>>(comps, (uint32_t)nc, cps, cpi, dx, sw);
         DBM_LAUNCH_CHECK();

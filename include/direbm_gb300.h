@@ -88,12 +88,12 @@ int dbm_disperse_f32(const float* d_pos_m, const float* d_f_m, int64_t m, int la
  * floor(y/cs)), stable radix sort, run-length encode, exclusive scan, sequential FP32 centroid
  * per run in sorted order.  d_cp_pos needs room for nc points; *p_out receives P (this call
  * synchronises the stream, as the reference's run_count.numpy() did).
- * The three functions below read the points' bounds back first, one short host wait each, to index them
- * with short keys; the refine leaves that out while its stream is being captured.  Their
- * temporaries come from a stream-ordered pool of the device that keeps up to 64 MB. */
+ * This function and dbm_resample_f32 read the points' bounds back first, one short host wait, to index
+ * them with short keys.  The temporaries of the three functions from here on come from a stream-ordered
+ * pool of the device that keeps up to 64 MB. */
 int dbm_create_control_points_f32(const float* d_pos_c, int64_t nc, float cs, float* d_cp_pos,
                                   int64_t* p_out, void* stream);
-/* refine_control_points: direbm/warp/propagation.py:77-112,249-275. */
+/* refine_control_points: direbm/warp/propagation.py:77-112,249-275.  Asynchronous. */
 int dbm_refine_control_points_f32(const float* d_cp_pos, int64_t p, const float* d_pos_c, const float* d_val_c,
                                   const int32_t* d_dir_c, int64_t nc, float dx, int kappa_hard,
                                   float* d_new_pos, void* stream);
