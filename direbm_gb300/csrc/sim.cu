@@ -998,8 +998,9 @@ __global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D,
   bool shared = false;  // the gather's blocks shared the directions and emitted nothing
   if constexpr (D == 2) shared = A.share_slots && direction_shares<Q>(*A.a.count, A.share_slots) > 1;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < Pn; j += gridDim.x * blockDim.x) {
-    const uint32_t em = A.emask[j];
-    if (only_gaps && !em && !shared) continue;  // emitted by the gather
+    const uint32_t emf = A.emask[j], em = emf & ~kEmitLater;
+    if (only_gaps && !emf && !shared) continue;  // emitted by the gather
+    if (emf != em) A.emask[j] = em;
     const uint32_t G = A.b.cell[j];
     const int b = find_instance(A.inst_base, A.n_inst, G);
     const InstK I = A.inst[b];

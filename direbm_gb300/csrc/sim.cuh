@@ -136,6 +136,9 @@ struct Args {
   int write_trace;
 };
 
+// Empty-mask bit of a control point that the gather left to k_emit although it emits the others itself.
+constexpr uint32_t kEmitLater = 1u << 31;
+
 // ---- geometry helpers ---------------------------------------------------------------------------
 
 __device__ __forceinline__ int find_instance(const uint32_t* __restrict__ base, int n, uint32_t g) {

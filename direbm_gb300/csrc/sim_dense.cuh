@@ -1042,30 +1042,24 @@ __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_GATHER) k_gather_ds(const _
   }
 }
 
-// A deferred tile's gather: clears its control points' empty masks, runs `gather`, and with fuse
-// emits the points that end up without an empty direction.
+// A deferred tile's gather: sets its control points' empty masks and runs `gather`.  With fuse the masks start
+// as kEmitLater, by which k_emit knows the points that nothing has emitted: emitting them here, from the sums
+// just written, cost the kernel its registers (1024 x 1024 cells at R = 1.9, most tiles deferred:
+// gather and emit 2583 us a step with it, 1683 without).
 template <int Q, class Fn>
 __device__ __forceinline__ void gather_fallback(const Args<Q, 2, PF32>& A, const Tile2& T, const InstK& I,
                                                 const TileGeo& G, bool fuse, Fn&& gather) {
   const int lx = threadIdx.x % G.tx, ly = threadIdx.x / G.tx;
-  uint32_t jb = 0, je = 0;  // this thread's cell's control points
   if (ly < G.ty && T.x0 + lx < I.dims[0] && T.y0 + ly < I.dims[1]) {
     const uint32_t g = I.base + (uint32_t)(T.x0 + lx) + (uint32_t)I.dims[0] * (uint32_t)(T.y0 + ly);
-    jb = A.b.start[g];
-    je = A.b.start[g + 1];
+    for (uint32_t j = A.b.start[g], je = A.b.start[g + 1]; j < je; ++j) A.emask[j] = fuse ? kEmitLater : 0u;
   }
-  for (uint32_t j = jb; j < je; ++j) A.emask[j] = 0u;
   __syncthreads();
   gather();
-  __syncthreads();
-  if (fuse)
-    for (uint32_t j = jb; j < je; ++j)
-      if (__ldcg(A.emask + j) == 0u) emit_from_cpf<Q>(A, (int)j);
 }
 
 // Row-segment passes over the deferred tiles (persistent grid; nothing to do when the list is
-// empty).  STAGE: 0 thin + refine, 1 weights, 2 gather (which first clears its control points' empty
-// masks and, with fuse, emits those that end up without an empty direction).
+// empty).  STAGE: 0 thin + refine, 1 weights, 2 gather.
 template <int Q, int STAGE>
 __global__ void __launch_bounds__(256) k_dense_fallback(const __grid_constant__ Args<Q, 2, PF32> A,
                                                        const Tile2* __restrict__ tiles, const TileGeo G,
