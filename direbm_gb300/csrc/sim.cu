@@ -2368,9 +2368,10 @@ struct SimImpl : SimBase {
     DBM_LAUNCH_CHECK();
     mark(4, s);
     if (upto <= 4) return DBM_OK;
-    // the dense gather writes every control point's empty mask and, unless the step keeps its
-    // intermediates, emits the points without an empty direction itself
-    const int fuse = ((dense && !split) || brick3_path()) && !A.write_trace ? 1 : 0;
+    // the dense gather writes every control point's empty mask and, with displacements of one cell or
+    // grid windows and unless the step keeps its intermediates, emits the points without an empty
+    // direction itself
+    const int fuse = ((dense && !split && (near_ok || grid_w)) || brick3_path()) && !A.write_trace ? 1 : 0;
     if (from_zero && !A.clear_emask) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (kTiles) {
       if (tiled_path()) {

@@ -264,6 +264,19 @@ __device__ __forceinline__ void stencil_axis(float p, float R, float tiny, int* 
   *lo = (int)floorf(p - R - tiny);
   *n = (int)floorf(p + R + tiny) - *lo + 1;
 }
+// Columns that a window's exact range can have: at most 3 up to R = 1, 4 up to 1.5, 5 up to 2 (less the
+// margins).  fn(integral constant) of that many.  Boxes with other displacements than one cell, or R < 1, take
+// each window by its exact range with them, a thread per point: as units of (point, direction) spread over the
+// block their sums left in scattered writes.  1024 x 1024 cells, one moment each, us a step, branching 4 x 4
+// stencil / units / now: dx 1, r 0.9 498 / 619 / 448; dx 1, r 0.7 477 / 621 / 447; dx 2, r 1.9 990 / 988 / 804.
+template <class Fn>
+__device__ __forceinline__ void with_columns(float R, float tiny, Fn&& fn) {
+  const float w = 2.f * (R + tiny) + 1e-4f;
+  if (w <= 2.f) fn(std::integral_constant<int, 3>{});
+  else if (w <= 3.f) fn(std::integral_constant<int, 4>{});
+  else fn(std::integral_constant<int, 5>{});
+}
+
 // Whether the 4 columns from `lo` hold every hit along one axis: the range is no wider, or it is five
 // wide (p within tiny of 1/2 at R = 1.5) and the fifth column's candidates, none of them nearer than
 // e5, all miss (rounding is monotone, so the smallest offset gives the smallest |e|).
@@ -528,7 +541,32 @@ __device__ __forceinline__ bool thin_refine_ds_tile(const Args<Q, 2, PF32>& A, c
       }
     }
   }
-  if (!fits) {
+  if (TX == 0 || (!fits && A.R > 1.55f)) {
+    with_columns(A.R, A.tiny, [&](auto nc) {
+      constexpr int NC = nc.value;
+      float cx[NC];
+#pragma unroll
+      for (int a = 0; a < NC; ++a) cx[a] = rn_sub((float)(jlx + a), cen[0]);
+#pragma unroll 1
+      for (int k = 0; k < Q; ++k) {
+        const int cdx = __float2int_rn(A.L.cdf[k][0]), cdy = __float2int_rn(A.L.cdf[k][1]);
+        const float2* o0 = S.xy() + (by + jly - cdy) * s2 + (bx + jlx - cdx);
+        const float* w0 = S.fl() + k * S.L.n1 + (by + jly - cdy) * s1 + (bx + jlx - cdx);
+        float dmin = 3.0e38f;
+#pragma unroll 1
+        for (int b = 0; b < nys; ++b, o0 += s2, w0 += s1) {
+          const float cyb = rn_sub((float)(jly + b), cen[1]);
+          float2 o[NC];
+#pragma unroll
+          for (int a = 0; a < NC; ++a) o[a] = a < nxs ? o0[a] : make_float2(kEmptyOff, kEmptyOff);
+#pragma unroll
+          for (int a = 0; a < NC; ++a) one(o[a], w0 + a, cx[a], cyb, dmin);
+        }
+        if (no) seconds(k, cdx, cdy, nys, nxs, dmin);
+        if (dmin <= A.R2) mask |= 1u << k;
+      }
+    });
+  } else if (!fits) {  // few points, and rows unrolled here would slow the others (R = 1.5: 118 -> 130 us)
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
       const int cdx = __float2int_rn(A.L.cdf[k][0]), cdy = __float2int_rn(A.L.cdf[k][1]);
@@ -552,8 +590,8 @@ __device__ __forceinline__ bool thin_refine_ds_tile(const Args<Q, 2, PF32>& A, c
 
 // ---- weights: per component, 1 / (sum over control points within R of (R - d)) -----------------
 
-// One component: direction k of a moment at offset o in region cell (bx, by).
-template <int Q, class SM>
+// One component: direction k of a moment at offset o in region cell (bx, by); NC: with_columns.
+template <int Q, int NC, class SM>
 __device__ __forceinline__ void weights_ds_unit(const Args<Q, 2, PF32>& A, const SM& S, int no, int m, int k,
                                                 int bx, int by) {
   const float2 o = make_float2(A.a.off[m], A.a.off[A.mcap + m]);
@@ -564,7 +602,7 @@ __device__ __forceinline__ void weights_ds_unit(const Args<Q, 2, PF32>& A, const
   const int cdx = __float2int_rn(A.L.cdf[k][0]), cdy = __float2int_rn(A.L.cdf[k][1]);
   const int row0 = by + uly + cdy, col0 = bx + ulx + cdx;
   CSum sws;
-  // branch-free, a row at a time (at most five columns for R < 2): a miss adds the weight 0
+  // branch-free, a row at a time: a miss adds the weight 0
   auto one = [&](float2 pc, float basex, float basey) {
     const float2 q = __fadd2_rn(make_float2(basex, basey), make_float2(-pc.x, -pc.y));
     const float2 e = __fadd2_rn(o, q);
@@ -574,11 +612,11 @@ __device__ __forceinline__ void weights_ds_unit(const Args<Q, 2, PF32>& A, const
 #pragma unroll 1
   for (int b = 0; b < nys; ++b) {
     const float2* row = S.xy() + (row0 + b) * S.L.s2 + col0;
-    float2 pc[5];
+    float2 pc[NC];
 #pragma unroll
-    for (int a = 0; a < 5; ++a) pc[a] = a < nxs ? row[a] : make_float2(kEmptyOff, kEmptyOff);
+    for (int a = 0; a < NC; ++a) pc[a] = a < nxs ? row[a] : make_float2(kEmptyOff, kEmptyOff);
 #pragma unroll
-    for (int a = 0; a < 5; ++a) one(pc[a], (float)(-(ulx + a)), (float)(-(uly + b)));
+    for (int a = 0; a < NC; ++a) one(pc[a], (float)(-(ulx + a)), (float)(-(uly + b)));
   }
   // then the second items, in window order
   uint64_t ov = no ? second_item_mask(S, no, row0, col0, nys, nxs) : 0u;
@@ -614,6 +652,15 @@ __device__ __forceinline__ bool weights_ds_tile(const Args<Q, 2, PF32>& A, const
   if (!dense) return false;
   const int no = *S.novf();  // second items in the overflow list (at most kOvf in a dense tile)
   if (!has) has = own.take(&m, &bx, &by);
+  if constexpr (TX == 0) {  // each thread its point's directions, windows by their exact ranges
+    with_columns(A.R, A.tiny, [&](auto nc) {
+#pragma unroll 1
+      for (; has; has = own.take(&m, &bx, &by))
+#pragma unroll 1
+        for (int k = 0; k < Q; ++k) weights_ds_unit<Q, nc.value>(A, S, no, m, k, bx, by);
+    });
+    return true;
+  }
   if (has) {
     bool fits = false;
     if constexpr (TX > 0) {
@@ -693,9 +740,9 @@ __device__ __forceinline__ bool weights_ds_tile(const Args<Q, 2, PF32>& A, const
   const int left = own.left();
 #pragma unroll 1
   for (int u = threadIdx.x; u < left * Q; u += blockDim.x) {
-    const int q = own.index(u / Q);
-    if (SPLIT && d2q9_cy(u % Q) != (int)blockIdx.y - 1) continue;
-    weights_ds_unit<Q>(A, S, no, own.item[q], u % Q, own.pos[q] & 0xffff, own.pos[q] >> 16);
+    const int k = u / left, q = own.index(u - k * left);
+    if (SPLIT && d2q9_cy(k) != (int)blockIdx.y - 1) continue;
+    weights_ds_unit<Q, 5>(A, S, no, own.item[q], k, own.pos[q] & 0xffff, own.pos[q] >> 16);
   }
   return true;
 }
@@ -725,8 +772,8 @@ __device__ __forceinline__ DF gather_total(float wf, float wlo, float hi, float 
   return df_add(df_mul(DF{wf, wlo}, df_norm(hi, lo)), DF{sb, 0.f});
 }
 
-// One (control point, direction): control point at offset pp in region cell (bx, by).
-template <int Q, class SM>
+// One (control point, direction): control point at offset pp in region cell (bx, by); NC: with_columns.
+template <int Q, int NC, class SM>
 __device__ __forceinline__ DF gather_ds_unit(const Args<Q, 2, PF32>& A, const SM& S, int no, float2 pp, int k,
                                              int bx, int by) {
   int jlx, nxs, jly, nys;
@@ -736,7 +783,7 @@ __device__ __forceinline__ DF gather_ds_unit(const Args<Q, 2, PF32>& A, const SM
   const int row0 = by + jly - cdy, col0 = bx + jlx - cdx;
   GatherSum s;
   s.clear();
-  // branch-free, a row at a time (at most five columns for R < 2): a miss gets the weight 0
+  // branch-free, a row at a time: a miss gets the weight 0
   auto one = [&](float2 o, float rho, float2 kv, float ex0, float ey0) {
     const float2 e = __fadd2_rn(o, make_float2(ex0, ey0));
     const float2 e2 = __fmul2_rn(e, e);
@@ -746,17 +793,17 @@ __device__ __forceinline__ DF gather_ds_unit(const Args<Q, 2, PF32>& A, const SM
   for (int b = 0; b < nys; ++b) {
     const float cyb = rn_sub((float)(jly + b), pp.y);
     const int i2 = (row0 + b) * S.L.s2 + col0, i1 = (row0 + b) * S.L.s1 + col0;
-    float2 o[5], kv[5];
-    float rho[5];
+    float2 o[NC], kv[NC];
+    float rho[NC];
 #pragma unroll
-    for (int a = 0; a < 5; ++a) {
+    for (int a = 0; a < NC; ++a) {
       const bool in = a < nxs;
       o[a] = in ? S.xy()[i2 + a] : make_float2(kEmptyOff, kEmptyOff);
       kv[a] = in ? S.kv()[k * S.L.n2 + i2 + a] : make_float2(0.f, 0.f);
       rho[a] = in ? S.fl()[i1 + a] : 0.f;
     }
 #pragma unroll
-    for (int a = 0; a < 5; ++a) one(o[a], rho[a], kv[a], rn_sub((float)(jlx + a), pp.x), cyb);
+    for (int a = 0; a < NC; ++a) one(o[a], rho[a], kv[a], rn_sub((float)(jlx + a), pp.x), cyb);
   }
   // then the second items, in window order
   uint64_t ov = no ? second_item_mask(S, no, row0, col0, nys, nxs) : 0u;
@@ -823,6 +870,24 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
   if (!dense) return false;
   const int no = *S.novf();  // second items in the overflow list (at most kOvf in a dense tile)
   if (!has) has = own.take(&j, &bx, &by);
+  if constexpr (TX == 0) {  // each thread its point's directions, windows by their exact ranges; no emit
+    with_columns(A.R, A.tiny, [&](auto nc) {
+#pragma unroll 1
+      for (; has; has = own.take(&j, &bx, &by)) {
+        const float2 pp = make_float2(A.b.off[j], A.b.off[A.ccap + j]);
+        uint32_t empty = 0;
+#pragma unroll 1
+        for (int k = 0; k < Q; ++k) {
+          const DF F = gather_ds_unit<Q, nc.value>(A, S, no, pp, k, bx, by);
+          A.cpfhi[(int64_t)k * A.ccap + j] = F.hi;
+          A.cpflo[(int64_t)k * A.ccap + j] = F.lo;
+          if (F.hi < A.eps) empty |= 1u << k;
+        }
+        A.emask[j] = empty;
+      }
+    });
+    return true;
+  }
   if (has) {
     bool fits = false;
     if constexpr (TX > 0) {
@@ -948,9 +1013,9 @@ __device__ __forceinline__ bool gather_ds_tile(const Args<Q, 2, PF32>& A, const 
   __syncthreads();
 #pragma unroll 1
   for (int u = threadIdx.x; u < left * Q; u += blockDim.x) {
-    const int e = u / Q, k = u - e * Q, q = own.index(e), i = own.item[q];
+    const int k = u / left, e = u - k * left, q = own.index(e), i = own.item[q];
     if (SPLIT && d2q9_cy(k) != (int)blockIdx.y - 1) continue;
-    const DF F = gather_ds_unit<Q>(A, S, no, make_float2(A.b.off[i], A.b.off[A.ccap + i]), k, own.pos[q] & 0xffff,
+    const DF F = gather_ds_unit<Q, 5>(A, S, no, make_float2(A.b.off[i], A.b.off[A.ccap + i]), k, own.pos[q] & 0xffff,
                                    own.pos[q] >> 16);
     A.cpfhi[(int64_t)k * A.ccap + i] = F.hi;
     A.cpflo[(int64_t)k * A.ccap + i] = F.lo;
@@ -1028,7 +1093,7 @@ __global__ void __launch_bounds__(256, DBM_DS_BLOCKS_WEIGHTS) k_weights_ds(const
 }
 
 template <int Q, int TX, bool SPLIT>
-__global__ void __launch_bounds__(256, DBM_DS_BLOCKS_GATHER) k_gather_ds(const __grid_constant__ Args<Q, 2, PF32> A,
+__global__ void __launch_bounds__(256, TX ? DBM_DS_BLOCKS_GATHER : 4) k_gather_ds(const __grid_constant__ Args<Q, 2, PF32> A,
                                                      const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
                                                      int* fb_tiles, int* fb_count, int fuse) {
   extern __shared__ __align__(16) unsigned char smem[];
