@@ -20,7 +20,7 @@ FP64, FP32DEV = 0, 1
 TRACE = {
     "occ": 1, "thin_cnt": 2, "centroid": 3, "mask": 4, "final_cell": 5, "final_off": 6,
     "sorted": 7, "sw": 8, "cpf": 9, "empty": 10, "fstar": 11, "counts": 12, "state_cell": 13, "state_off": 14,
-    "import_order": 15,
+    "import_order": 15, "deferred": 16,
 }
 
 # Arrays of a recorded step (dbm_tape_export): name -> (id, dtype, shape kind).  Shape kinds: "M",

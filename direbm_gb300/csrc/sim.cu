@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) k_collide(const __grid_constant__ Args<Q,
         A.a.dev[(int64_t)k * A.mcap + m] = dv[k];
         big = __fadd_rn(big, fabsf(dv[k]));
       }
-      if (A.odd_f && !(A.a.rho[m] >= 0.f && big < 3.4e38f)) *A.odd_f = 1;
+      if (A.odd_f && !(A.a.rho[m] >= 0.f && big < 3.4e38f)) A.odd_f[b] = 1;
       if (A.want_wexp) {
         const float rho = A.a.rho[m];
 #pragma unroll
@@ -1454,7 +1454,8 @@ struct SimImpl : SimBase {
   TileGeo geo_s{};
   size_t sm_gather_s = 0;
   // dense-stencil kernels (k_*_ds, shared memory = the dense layout) and the list of tiles they
-  // defer to the row-segment code: d_fb[0..2] the per-stage counts, d_fb + 4 the tile indices
+  // defer to the row-segment code: d_fb[0..2] the per-stage counts, from [4] on odd_f per instance, from
+  // fb_head() on the tile indices
   bool near_ok = false;         // their NEAR variants apply (dx = cell, D2Q9, 1 <= R < 2)
   size_t sm_ds[3] = {0, 0, 0};  // thin+refine, weights, gather
   // grid kernels (k_*_grid): window width W in cells they are compiled for, 0 where they do not apply
@@ -1466,11 +1467,12 @@ struct SimImpl : SimBase {
   int split_ds[3] = {1, 1, 1};    // blocks per tile, dense kernels
   int* d_fb = nullptr;
   // 3D grid kernels (k_brick3): bricks of 8^3 cells away from obstacles, the other bricks (8 x 8 x 4, for
-  // the untiled kernels), and per stage the bricks they defer (d_fb3[0..2] counts, [3] odd_f, + 4 list)
+  // the untiled kernels), and per stage the bricks they defer (d_fb3, laid out as d_fb)
   bool brick3_ok = false;
   Brick *d_bricks3 = nullptr, *d_near3 = nullptr;
   int nbricks3 = 0, nnear3 = 0;
   int* d_fb3 = nullptr;
+  int fb_head() const { return 4 + (int)inst_h.size(); }
   int use_persistent = 0;
   TileGeo geo{};
   size_t sm_refine = 0, sm_weights = 0, sm_gather = 0;
@@ -1725,7 +1727,7 @@ struct SimImpl : SimBase {
       if (!d_bricks3) {  // at creation, with every brick clear
         DBM_TRY(alloc(&d_bricks3, (int64_t)far.size()));
         DBM_TRY(alloc(&d_near3, 2 * (int64_t)far.size()));
-        DBM_TRY(alloc(&d_fb3, (int64_t)far.size() + 4));
+        DBM_TRY(alloc(&d_fb3, (int64_t)far.size() + fb_head()));
       }
       if (own) DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the old lists
       DBM_CUDA(cudaMemcpy(d_bricks3, far.data(), sizeof(Brick) * far.size(), cudaMemcpyHostToDevice));
@@ -1745,10 +1747,10 @@ struct SimImpl : SimBase {
       const BrickGeo half{kBrick3, kBrick3, kBrick3 / 2};
       if (nbricks3 > 0) {
         constexpr int smem = grid3_layout(STAGE).total;
-        k_brick3<Q, STAGE><<<nbricks3, kThreads3, smem, s>>>(A, d_bricks3, nbricks3, d_fb3 + 4, d_fb3 + STAGE, fuse);
+        k_brick3<Q, STAGE><<<nbricks3, kThreads3, smem, s>>>(A, d_bricks3, nbricks3, d_fb3 + fb_head(), d_fb3 + STAGE, fuse);
         DBM_LAUNCH_CHECK();
         const unsigned gf = (unsigned)std::min<int64_t>((int64_t)nbricks3 * (STAGE == 0 ? 2 : 2 * Q), sm_count() * 6);
-        k_brick3_fallback<Q, STAGE><<<gf, 256, 0, s>>>(A, d_bricks3, d_fb3 + 4, d_fb3 + STAGE);
+        k_brick3_fallback<Q, STAGE><<<gf, 256, 0, s>>>(A, d_bricks3, d_fb3 + fb_head(), d_fb3 + STAGE);
         DBM_LAUNCH_CHECK();
       }
       if (nnear3 > 0) {
@@ -1760,7 +1762,7 @@ struct SimImpl : SimBase {
       if (STAGE == 2 && fuse) {
         if (nbricks3 > 0) {
           const unsigned ge = (unsigned)std::min<int64_t>((int64_t)nbricks3 * 2, sm_count() * 4);
-          k_emit_bricks<Q><<<ge, 256, 0, s>>>(A, d_bricks3, half, nbricks3, d_fb3 + 4, d_fb3 + STAGE);
+          k_emit_bricks<Q><<<ge, 256, 0, s>>>(A, d_bricks3, half, nbricks3, d_fb3 + fb_head(), d_fb3 + STAGE);
           DBM_LAUNCH_CHECK();
         }
         if (nnear3 > 0) {
@@ -1949,8 +1951,8 @@ struct SimImpl : SimBase {
       d_fb = nullptr;
     }
     if (shift_ok || grid_w) {
-      DBM_TRY(alloc(&d_fb, (int64_t)ntiles + 4));
-      DBM_CUDA(cudaMemset(d_fb, 0, ((size_t)ntiles + 4) * sizeof(int)));
+      DBM_TRY(alloc(&d_fb, (int64_t)ntiles + fb_head()));
+      DBM_CUDA(cudaMemset(d_fb, 0, ((size_t)ntiles + fb_head()) * sizeof(int)));
     }
     if constexpr (kTiles) {
       DBM_CUDA(cudaFuncSetAttribute((const void*)k_thin_refine_t<Q, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2229,8 +2231,8 @@ struct SimImpl : SimBase {
     A.want_wexp = untiled ? 1 : 0;
     // fallback counts of the three stages, odd_f
     int* const fb = brick3_path() ? d_fb3 : d_fb;
-    A.odd_f = fb ? fb + 3 : nullptr;
-    if (fb) DBM_CUDA(cudaMemsetAsync(fb, 0, 4 * sizeof(int), s));
+    A.odd_f = fb ? fb + 4 : nullptr;
+    if (fb) DBM_CUDA(cudaMemsetAsync(fb, 0, (size_t)fb_head() * sizeof(int), s));
     // the gather's empty masks: written whole by one block per tile, else combined from zero
     bool dense = false, split = false, shared = false;  // shared: split if the device says so
     if constexpr (kTiles) {
@@ -2259,18 +2261,18 @@ struct SimImpl : SimBase {
         if (shift_ok && use_shift && use_dense) {
           const int grid = use_persistent ? pgrid_ds[0] : ntiles;
           with_near([&](auto tx) {
-            k_thin_refine_ds<Q, tx.value><<<grid, 256, sm_ds[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
+            k_thin_refine_ds<Q, tx.value><<<grid, 256, sm_ds[0], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 0);
           });
           DBM_LAUNCH_CHECK();
-          k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
+          k_dense_fallback<Q, 0><<<pgrid_rs, 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 0, 0);
           shifted = true;
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[0] : ntiles;
           with_grid([&](auto w) {
-            k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 0);
+            k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 0);
           });
           DBM_LAUNCH_CHECK();
-          k_grid_fallback<Q, 0><<<pgrid[0], 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 0, 0);
+          k_grid_fallback<Q, 0><<<pgrid[0], 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 0, 0);
           shifted = true;
         } else if (shift_ok && use_shift) {
           k_thin_refine_t<Q, P, true><<<use_persistent ? pgrid_rs : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo,
@@ -2336,19 +2338,19 @@ struct SimImpl : SimBase {
             if constexpr (Q == 9 && tx.value == 32)
               if (split_ds[1] > 1)
                 return k_weights_ds<Q, 32, true><<<dim3(grid, 3), 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles,
-                                                                                      d_fb + 4, d_fb + 1);
-            k_weights_ds<Q, tx.value, false><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+                                                                                      d_fb + fb_head(), d_fb + 1);
+            k_weights_ds<Q, tx.value, false><<<grid, 256, sm_ds[1], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 1);
           });
           DBM_LAUNCH_CHECK();
-          k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
+          k_dense_fallback<Q, 1><<<pgrid_ws, 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 1, 0);
           shifted = true;
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[1] : ntiles;
           with_grid([&](auto w) {
-            k_weights_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 1);
+            k_weights_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 1);
           });
           DBM_LAUNCH_CHECK();
-          k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 1, 0);
+          k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 1, 0);
           shifted = true;
         } else if (shift_ok && use_shift) {
           k_weights_t<Q, P, true><<<use_persistent ? pgrid_ws : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo,
@@ -2382,20 +2384,20 @@ struct SimImpl : SimBase {
             if constexpr (Q == 9 && tx.value == 32)
               if (split_ds[2] > 1)
                 return k_gather_ds<Q, 32, true><<<dim3(grid, 3), 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles,
-                                                                                     d_fb + 4, d_fb + 2, fuse);
-            k_gather_ds<Q, tx.value, false><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + 4, d_fb + 2,
+                                                                                     d_fb + fb_head(), d_fb + 2, fuse);
+            k_gather_ds<Q, tx.value, false><<<grid, 256, sm_ds[2], s>>>(A, d_tiles, geo_s, ntiles, d_fb + fb_head(), d_fb + 2,
                                                                         fuse);
           });
           DBM_LAUNCH_CHECK();
-          k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + 4, d_fb + 2, fuse);
+          k_dense_fallback<Q, 2><<<pgrid_s, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, d_fb + fb_head(), d_fb + 2, fuse);
           shifted = true;
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[2] : ntiles;
           with_grid([&](auto w) {
-            k_gather_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + 4, d_fb + 2, fuse);
+            k_gather_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 2, fuse);
           });
           DBM_LAUNCH_CHECK();
-          k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + 4, d_fb + 2, fuse);
+          k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 2, fuse);
           shifted = true;
         } else if (shift_ok && use_shift) {
           k_gather_ts<Q><<<use_persistent ? pgrid_s : ntiles, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, ntiles);
@@ -2774,6 +2776,16 @@ struct SimImpl : SimBase {
           if (nbytes < sz) { set_last_error("trace: destination too small"); return DBM_ERR_INVALID; }
           DBM_CUDA(cudaMemcpyAsync(dst, A.a.count, 4, cudaMemcpyDeviceToDevice, s));
           DBM_CUDA(cudaMemcpyAsync((char*)dst + 4, A.d_P, 4, cudaMemcpyDeviceToDevice, s));
+        }
+        return DBM_OK;
+      }
+      case DBM_TRACE_DEFERRED: {
+        const int* fb = brick3_path() ? d_fb3 : d_fb;
+        if (needed) *needed = 12;
+        if (dst) {
+          if (nbytes < 12) { set_last_error("trace: destination too small"); return DBM_ERR_INVALID; }
+          if (fb) DBM_CUDA(cudaMemcpyAsync(dst, fb, 12, cudaMemcpyDeviceToDevice, s));
+          else DBM_CUDA(cudaMemsetAsync(dst, 0, 12, s));
         }
         return DBM_OK;
       }

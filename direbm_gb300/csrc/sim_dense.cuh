@@ -26,7 +26,7 @@
 // ascending, then columns ascending), then the second items in the same cell order.  A tile whose
 // region holds a cell with three or more items, or more two-item cells than the overflow list takes,
 // is handed to the row-segment code (a second, normally empty, launch over the deferred tiles); so
-// are all tiles of the gather when a density is negative or an f is not finite (0 x it is not 0).
+// are the gather's tiles of an instance with a negative density or an f that is not finite (0 x it is not 0).
 //
 // Bound by instruction issue (thin + refine 88 % of issue slots and 87 % of shared-memory wavefronts,
 // weights 78 %, gather 70 %; DRAM 5-10 %).  Ensemble of 15.5 M moments, 16 x 16 tiles, ms per step,
@@ -1100,8 +1100,8 @@ __global__ void __launch_bounds__(256, TX ? DBM_DS_BLOCKS_GATHER : 4) k_gather_d
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
-    // a negative density or an f that is not finite anywhere (noted by the collision): no dense tile
-    if ((*A.odd_f || !gather_ds_tile<Q, TX, SPLIT>(A, T, I, G, fuse != 0, smem)) && (!SPLIT || blockIdx.y == 0))
+    // a negative density or an f that is not finite in the instance (noted by the collision): no dense tile
+    if ((A.odd_f[T.inst] || !gather_ds_tile<Q, TX, SPLIT>(A, T, I, G, fuse != 0, smem)) && (!SPLIT || blockIdx.y == 0))
       defer_tile(tb, fb_tiles, fb_count);
     __syncthreads();
   }

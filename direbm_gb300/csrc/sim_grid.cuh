@@ -586,8 +586,8 @@ __global__ void __launch_bounds__(256, 4) k_gather_grid(const __grid_constant__ 
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
-    // a negative density or an f that is not finite anywhere (noted by the collision): no grid tile
-    if ((*A.odd_f || !gather_grid_tile<Q, W>(A, T, I, G, shares, fuse != 0, smem)) && blockIdx.y == 0)
+    // a negative density or an f that is not finite in the instance (noted by the collision): no grid tile
+    if ((A.odd_f[T.inst] || !gather_grid_tile<Q, W>(A, T, I, G, shares, fuse != 0, smem)) && blockIdx.y == 0)
       defer_tile(tb, fb_tiles, fb_count);
     __syncthreads();
   }

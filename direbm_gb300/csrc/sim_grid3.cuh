@@ -16,8 +16,8 @@
 // some lane meets a marked row looks for them after each candidate of that row.  The sums of weights are
 // exact, so the weights kernel visits them at the end.  Results are bit-identical to the untiled kernels.  Bricks within reach of an
 // obstacle's bounced components are not taken (the host leaves them to the untiled kernels), and bricks
-// with more further items than the list takes are deferred to them, as are all bricks of the gather when
-// a density is negative or an f is not finite.
+// with more further items than the list takes are deferred to them, as are the gather's bricks of an
+// instance with a negative density or an f that is not finite.
 // Bound by instruction issue (72 - 88 % of slots) and shared-memory wavefronts (71 - 87 %).  D3Q19, 96^3
 // cells with one moment each, ms per launch, untiled / grid: thin + refine 2.97 / 1.13, weights 2.53 /
 // 1.02, gather with emit 3.62 / 1.58; after 100 steps (0.4 % of the cells with two items) 2.99 / 1.55,
@@ -619,8 +619,8 @@ __global__ void __launch_bounds__(kThreads3, 2) k_brick3(const __grid_constant__
     bool ok;
     if constexpr (STAGE == 0) ok = thin_refine_brick<Q>(A, B, I, smem);
     else if constexpr (STAGE == 1) ok = weights_brick<Q>(A, B, I, smem);
-    // a negative density or an f that is not finite anywhere (noted by the collision): no brick
-    else ok = !*A.odd_f && gather_brick<Q>(A, B, I, fuse != 0, smem);
+    // a negative density or an f that is not finite in the instance (noted by the collision): no brick
+    else ok = !A.odd_f[B.inst] && gather_brick<Q>(A, B, I, fuse != 0, smem);
     if (!ok && threadIdx.x == 0) fb_bricks[atomicAdd(fb_count, 1)] = bi;
     __syncthreads();
   }

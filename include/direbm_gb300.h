@@ -353,6 +353,8 @@ int dbm_tape_export(dbm_tape* tape, int32_t index, int32_t what, void* d_dst, in
 #define DBM_TRACE_STATE_OFF 14  /* real[D][Mcap] offsets of each current moment */
 #define DBM_TRACE_IMPORT_ORDER 15 /* u32[Mcap] after dbm_sim_set_state (and before any step):
                                      input index of each sorted moment */
+#define DBM_TRACE_DEFERRED 16  /* u32[3] tiles (2D) or bricks (3D) of the last step's thin + refine, weights
+                                  and gather that the dense or grid kernels left to the general ones */
 
 #ifdef __cplusplus
 }
