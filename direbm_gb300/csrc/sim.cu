@@ -1442,6 +1442,8 @@ struct SimImpl : SimBase {
   cudaGraphExec_t graph_tr[2] = {nullptr, nullptr};  // the same step writing every intermediate
   unsigned long long graph_kernels = 0, graph_tr_kernels = 0;
   int trace_on = 0;
+  // the last step's gather left all its sums in memory (DBM_TRACE_CPF); graph_cpf: a captured step does
+  bool cpf_whole = true, graph_cpf = true;
   // shared-memory tiling (2D)
   bool tiled = false;
   Tile2* d_tiles = nullptr;
@@ -2374,6 +2376,7 @@ struct SimImpl : SimBase {
     // grid windows and unless the step keeps its intermediates, emits the points without an empty
     // direction itself
     const int fuse = ((dense && !split && (near_ok || grid_w)) || brick3_path()) && !A.write_trace ? 1 : 0;
+    cpf_whole = !fuse;
     if (from_zero && !A.clear_emask) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (kTiles) {
       if (tiled_path()) {
@@ -2438,11 +2441,13 @@ struct SimImpl : SimBase {
           if (rc != DBM_OK) return rc;
           if (e != cudaSuccess) { set_last_error("graph capture failed: %s", cudaGetErrorString(e)); return DBM_ERR_CUDA; }
           graph_kernels = g_launches - before;
+          graph_cpf = cpf_whole;
           g_launches = before;
           DBM_CUDA(cudaGraphInstantiate(&graph[cur], gr, 0));
           cudaGraphDestroy(gr);
         }
         DBM_CUDA(cudaGraphLaunch(graph[cur], own));
+        cpf_whole = graph_cpf;
         count_launch(graph_kernels);
       } else {
         DBM_TRY(launch_step(own, 99));
@@ -2743,6 +2748,10 @@ struct SimImpl : SimBase {
       case DBM_TRACE_CPF:
         if constexpr (std::is_same<P, PF64>::value) { src = A.cpf64; sz = (int64_t)Q * ccap * 8; }
         else {
+          if (!cpf_whole) {  // the gather emitted most points from registers: what is there is of older steps
+            set_last_error("trace: a plain step keeps no gathered f (dbm_sim_step_partial does)");
+            return DBM_ERR_STATE;
+          }
           sz = (int64_t)2 * Q * ccap * 4;
           if (needed) *needed = sz;
           if (dst) {
