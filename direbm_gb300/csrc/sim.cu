@@ -1462,6 +1462,7 @@ struct SimImpl : SimBase {
   size_t sm_ds[3] = {0, 0, 0};  // thin+refine, weights, gather
   // grid kernels (k_*_grid): window width W in cells they are compiled for, 0 where they do not apply
   int grid_w = 0;
+  TileGeo geo_g{};  // geo with the staging capacities of the row segments in their blocks
   size_t sm_grid[3] = {0, 0, 0};
   int pgrid_grid[3] = {1, 1, 1};
   int pgrid_ds[3] = {1, 1, 1};
@@ -1936,6 +1937,14 @@ struct SimImpl : SimBase {
         sm_grid[i] = (size_t)L.total;
         if (sm_grid[i] > 200 * 1024 || L.rw >= 4096 || L.rh >= 2048) grid_w = 0;  // the list's keys hold 12 + 11 bits
       }
+      // the row segments run in the grid kernels' blocks: four of them, with their lists, on an SM
+      const size_t seg = 53 * 1024;
+      geo_g = geo;
+      geo_g.cap_refine = pick_cap(0, mcells, seg);
+      geo_g.cap_weights = pick_cap(1, ccells, seg);
+      geo_g.cap_gather = pick_cap(2, mcells, seg);
+      const int cap[3] = {geo_g.cap_refine, geo_g.cap_weights, geo_g.cap_gather};
+      for (int i = 0; i < 3; ++i) sm_grid[i] = std::max(sm_grid[i], smem_for(i, cap[i]));
     }
     std::vector<Tile2> tiles;
     for (int i = 0; i < (int)inst_h.size(); ++i)
@@ -1975,13 +1984,9 @@ struct SimImpl : SimBase {
           kg[1] = (const void*)k_weights_grid<Q, w.value>;
           kg[2] = (const void*)k_gather_grid<Q, w.value>;
         });
-        const void* kf[3] = {(const void*)k_grid_fallback<Q, 0>, (const void*)k_grid_fallback<Q, 1>,
-                             (const void*)k_grid_fallback<Q, 2>};
-        const size_t sf[3] = {sm_refine, sm_weights, sm_gather};
         int slots = 1 << 30;
         for (int i = 0; i < 3; ++i) {
           DBM_CUDA(cudaFuncSetAttribute(kg[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_grid[i]));
-          DBM_CUDA(cudaFuncSetAttribute(kf[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf[i]));
           int nbd = 1;
           DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kg[i], 256, sm_grid[i]));
           pgrid_grid[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
@@ -2271,10 +2276,9 @@ struct SimImpl : SimBase {
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[0] : ntiles;
           with_grid([&](auto w) {
-            k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 0);
+            k_thin_refine_grid<Q, w.value><<<grid, 256, sm_grid[0], s>>>(A, d_tiles, geo_g, ntiles, d_fb + 0);
           });
           DBM_LAUNCH_CHECK();
-          k_grid_fallback<Q, 0><<<pgrid[0], 256, sm_refine, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 0, 0);
           shifted = true;
         } else if (shift_ok && use_shift) {
           k_thin_refine_t<Q, P, true><<<use_persistent ? pgrid_rs : ntiles, 256, sm_refine, s>>>(A, d_tiles, geo,
@@ -2349,10 +2353,9 @@ struct SimImpl : SimBase {
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[1] : ntiles;
           with_grid([&](auto w) {
-            k_weights_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[1], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 1);
+            k_weights_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[1], s>>>(A, d_tiles, geo_g, ntiles, d_fb + 1);
           });
           DBM_LAUNCH_CHECK();
-          k_grid_fallback<Q, 1><<<pgrid[1], 256, sm_weights, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 1, 0);
           shifted = true;
         } else if (shift_ok && use_shift) {
           k_weights_t<Q, P, true><<<use_persistent ? pgrid_ws : ntiles, 256, sm_weights, s>>>(A, d_tiles, geo,
@@ -2397,10 +2400,9 @@ struct SimImpl : SimBase {
         } else if (grid_path()) {
           const int grid = use_persistent ? pgrid_grid[2] : ntiles;
           with_grid([&](auto w) {
-            k_gather_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[2], s>>>(A, d_tiles, geo, ntiles, d_fb + fb_head(), d_fb + 2, fuse);
+            k_gather_grid<Q, w.value><<<dim3(grid, grid_y), 256, sm_grid[2], s>>>(A, d_tiles, geo_g, ntiles, d_fb + 2, fuse);
           });
           DBM_LAUNCH_CHECK();
-          k_grid_fallback<Q, 2><<<pgrid[2], 256, sm_gather, s>>>(A, d_tiles, geo, d_fb + fb_head(), d_fb + 2, fuse);
           shifted = true;
         } else if (shift_ok && use_shift) {
           k_gather_ts<Q><<<use_persistent ? pgrid_s : ntiles, 256, sm_gather_s, s>>>(A, d_tiles, geo_s, ntiles);

@@ -16,7 +16,7 @@
 // All further items of the region's cells are kept in one list ordered by (row, column, place in the
 // cell); after a direction's grid pass the window's part of the list follows, in that order, which is
 // the row-segment kernels' second pass.  Results are bit-identical to them.  A tile with more further
-// items than the list takes is handed to the row-segment code (k_grid_fallback, normally empty).
+// items than the list takes goes to the row-segment code, in the same block.
 // Bound by instruction issue.  D2Q7, R = 4, 368,640 moments, one per cell, us per launch, row segments /
 // grid: thin + refine 828 / 155, weights 371 / 171, gather 1098 / 255, whole step 2490 / 641; after 100
 // steps (two-item cells) 3333 / 744.
@@ -541,22 +541,35 @@ __device__ __forceinline__ bool gather_grid_tile(const Args<Q, 2, PF32>& A, cons
 // (direction_shares): as many as the blocks of the moments' tiles (256 cells, one moment each where the store is full) still run at once, and
 // the directions in equal parts.  The gather then leaves its sums to the emit pass.  D2Q7 at R = 4
 // cells, 5 k to 30 k moments in 24 k to 63 k cells: weights 93 -> 33 us, gather 167 -> 47.  Every block of a tile
-// stages the same items and finds the same fault, and the first defers it.
+// stages the same items and finds the same fault, and the first takes it to the row segments.
+
+__device__ __forceinline__ void count_deferred(int* fb_count) {
+  if (threadIdx.x == 0) atomicAdd(fb_count, 1);
+}
+
 // This launch's shares (the moments the step began with); slots 0: one.
 template <int Q>
 __device__ __forceinline__ int grid_shares(const Args<Q, 2, PF32>& A) {
   return A.share_slots ? min(direction_shares<Q>(*A.a.count, A.share_slots), (int)gridDim.y) : 1;
 }
 
+
+// A tile that cannot be staged goes to the row-segment code at once, in the same block (and shared memory,
+// of the larger need): its few tiles are the last to finish, and in a launch of their own they started after
+// all others had (a cluster in 512 x 512 cells, 57 k moments, R = 1.5: 545 -> 387 us a step, row segments alone
+// 416; R = 4: 1689 -> 1357, 1407).  fb_count: their number.
 template <int Q, int W>
 __global__ void __launch_bounds__(256, 4) k_thin_refine_grid(const __grid_constant__ Args<Q, 2, PF32> A,
                                                             const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
-                                                            int* fb_tiles, int* fb_count) {
+                                                            int* fb_count) {
   extern __shared__ __align__(16) unsigned char smem[];
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
-    if (!thin_refine_grid_tile<Q, W>(A, T, I, G, smem)) defer_tile(tb, fb_tiles, fb_count);
+    if (!thin_refine_grid_tile<Q, W>(A, T, I, G, smem)) {
+      count_deferred(fb_count);
+      thin_refine_tile<Q, PF32, false>(A, T, I, G, smem);
+    }
     __syncthreads();
   }
 }
@@ -564,14 +577,17 @@ __global__ void __launch_bounds__(256, 4) k_thin_refine_grid(const __grid_consta
 template <int Q, int W>
 __global__ void __launch_bounds__(256, 4) k_weights_grid(const __grid_constant__ Args<Q, 2, PF32> A,
                                                         const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
-                                                        int* fb_tiles, int* fb_count) {
+                                                        int* fb_count) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int shares = grid_shares<Q>(A);
   if ((int)blockIdx.y >= shares) return;
   for (int tb = blockIdx.x; tb < ntiles; tb += gridDim.x) {
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
-    if (!weights_grid_tile<Q, W>(A, T, I, G, shares, smem) && blockIdx.y == 0) defer_tile(tb, fb_tiles, fb_count);
+    if (!weights_grid_tile<Q, W>(A, T, I, G, shares, smem) && blockIdx.y == 0) {
+      count_deferred(fb_count);
+      weights_tile<Q, PF32, false>(A, T, I, G, smem);
+    }
     __syncthreads();
   }
 }
@@ -579,7 +595,7 @@ __global__ void __launch_bounds__(256, 4) k_weights_grid(const __grid_constant__
 template <int Q, int W>
 __global__ void __launch_bounds__(256, 4) k_gather_grid(const __grid_constant__ Args<Q, 2, PF32> A,
                                                        const Tile2* __restrict__ tiles, const TileGeo G, int ntiles,
-                                                       int* fb_tiles, int* fb_count, int fuse) {
+                                                       int* fb_count, int fuse) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int shares = grid_shares<Q>(A);
   if ((int)blockIdx.y >= shares) return;
@@ -587,28 +603,8 @@ __global__ void __launch_bounds__(256, 4) k_gather_grid(const __grid_constant__ 
     const Tile2 T = tiles[tb];
     const InstK I = A.inst[T.inst];
     // a negative density or an f that is not finite in the instance (noted by the collision): no grid tile
-    if ((A.odd_f[T.inst] || !gather_grid_tile<Q, W>(A, T, I, G, shares, fuse != 0, smem)) && blockIdx.y == 0)
-      defer_tile(tb, fb_tiles, fb_count);
-    __syncthreads();
-  }
-}
-
-// Row-segment passes over the deferred tiles, as k_dense_fallback, with the windows of each direction.
-template <int Q, int STAGE>
-__global__ void __launch_bounds__(256) k_grid_fallback(const __grid_constant__ Args<Q, 2, PF32> A,
-                                                      const Tile2* __restrict__ tiles, const TileGeo G,
-                                                      const int* __restrict__ fb_tiles,
-                                                      const int* __restrict__ fb_count, int fuse) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int n = *fb_count;
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const Tile2 T = tiles[fb_tiles[i]];
-    const InstK I = A.inst[T.inst];
-    if constexpr (STAGE == 0) {
-      thin_refine_tile<Q, PF32, false>(A, T, I, G, smem);
-    } else if constexpr (STAGE == 1) {
-      weights_tile<Q, PF32, false>(A, T, I, G, smem);
-    } else {
+    if ((A.odd_f[T.inst] || !gather_grid_tile<Q, W>(A, T, I, G, shares, fuse != 0, smem)) && blockIdx.y == 0) {
+      count_deferred(fb_count);
       gather_fallback<Q>(A, T, I, G, fuse != 0, [&] { gather_tile<Q, PF32>(A, T, I, G, smem); });
     }
     __syncthreads();
