@@ -39,8 +39,10 @@ __global__ void __launch_bounds__(256) k_collide(const __grid_constant__ Args<Q,
   if (A.clear_start)
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= A.ncells; c += gridDim.x * blockDim.x)
       A.b.start[c] = 0u;
+  int further = 0;  // moments of this thread beyond the first of their cells
   for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
     const uint32_t g = A.a.cell[m];
+    if (D == 3 && A.further && m > 0 && A.a.cell[m - 1] == g) ++further;
     const int b = find_instance(A.inst_base, A.n_inst, g);
     const InstK I = A.inst[b];
     int c[3] = {0, 0, 0};
@@ -122,6 +124,10 @@ __global__ void __launch_bounds__(256) k_collide(const __grid_constant__ Args<Q,
       }
       if (out) atomicOr(A.status, ST_OUT_OF_BOX);
     }
+  }
+  if (D == 3 && A.further) {
+    const int sum = __reduce_add_sync(0xffffffffu, further);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(A.further, sum);
   }
 }
 
@@ -995,8 +1001,9 @@ template <int Q, int D, class P>
 __global__ void __launch_bounds__(256) k_emit(const __grid_constant__ Args<Q, D, P> A, int only_gaps) {
   using real = typename P::real;
   const uint32_t Pn = *A.d_P;
-  bool shared = false;  // the gather's blocks shared the directions and emitted nothing
+  bool shared = false;  // the gather emitted nothing: its blocks shared the directions, or a crowded 3D state
   if constexpr (D == 2) shared = A.share_slots && direction_shares<Q>(*A.a.count, A.share_slots) > 1;
+  else shared = A.further && (int64_t)*A.further * 32 > (int64_t)*A.a.count;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < Pn; j += gridDim.x * blockDim.x) {
     const uint32_t emf = A.emask[j], em = emf & ~kEmitLater;
     if (only_gaps && !emf && !shared) continue;  // emitted by the gather
@@ -1466,8 +1473,9 @@ struct SimImpl : SimBase {
   TileGeo geo_s{};
   size_t sm_gather_s = 0;
   // dense-stencil kernels (k_*_ds, shared memory = the dense layout) and the list of tiles they
-  // defer to the row-segment code: d_fb[0..2] the per-stage counts, from [4] on odd_f per instance, from
-  // fb_head() on the tile indices
+  // defer to the row-segment code: d_fb[0..2] the per-stage counts, [3] `further`, [4..6] tickets (3D), from
+  // kFbFlags on odd_f per instance, from fb_head() on the tile indices
+  static constexpr int kFbFlags = 8;
   bool near_ok = false;         // their NEAR variants apply (dx = cell, D2Q9, 1 <= R < 2)
   size_t sm_ds[3] = {0, 0, 0};  // thin+refine, weights, gather
   // grid kernels (k_*_grid): window width W in cells they are compiled for, 0 where they do not apply
@@ -1484,8 +1492,9 @@ struct SimImpl : SimBase {
   bool brick3_ok = false;
   Brick *d_bricks3 = nullptr, *d_near3 = nullptr;
   int nbricks3 = 0, nnear3 = 0;
+  int brick3_y = 1;               // blocks per brick (weights, gather)
   int* d_fb3 = nullptr;
-  int fb_head() const { return 4 + (int)inst_h.size(); }
+  int fb_head() const { return kFbFlags + (int)inst_h.size(); }
   int use_persistent = 0;
   TileGeo geo{};
   size_t sm_refine = 0, sm_weights = 0, sm_gather = 0;
@@ -1748,6 +1757,7 @@ struct SimImpl : SimBase {
       if (nbricks3 != (int)far.size() || nnear3 != (int)near.size()) invalidate_graphs();  // launches hold the sizes
       nbricks3 = (int)far.size();
       nnear3 = (int)near.size();
+      brick3_y = std::max(1, std::min(Q, 2 * sm_count() / std::max(nbricks3, 1)));  // two blocks run on an SM
     }
     return DBM_OK;
   }
@@ -1762,12 +1772,14 @@ struct SimImpl : SimBase {
   int launch_brick3(Args<Q, D, P>& A, int fuse, cudaStream_t s) {
     if constexpr (D == 3 && std::is_same<P, PF32>::value) {
       const BrickGeo half{kBrick3, kBrick3, kBrick3 / 2};
+      int* const list = d_fb3 + fb_head();
       if (nbricks3 > 0) {
         constexpr int smem = grid3_layout(STAGE).total;
-        k_brick3<Q, STAGE><<<nbricks3, kThreads3, smem, s>>>(A, d_bricks3, nbricks3, d_fb3 + fb_head(), d_fb3 + STAGE, fuse);
+        const unsigned grid = (unsigned)nbricks3 * (STAGE == 0 ? 1 : brick3_y);
+        k_brick3<Q, STAGE><<<grid, kThreads3, smem, s>>>(A, d_bricks3, nbricks3, list, d_fb3 + STAGE, fuse);
         DBM_LAUNCH_CHECK();
         const unsigned gf = (unsigned)std::min<int64_t>((int64_t)nbricks3 * (STAGE == 0 ? 2 : 2 * Q), sm_count() * 6);
-        k_brick3_fallback<Q, STAGE><<<gf, 256, 0, s>>>(A, d_bricks3, d_fb3 + fb_head(), d_fb3 + STAGE);
+        k_brick3_fallback<Q, STAGE><<<gf, 256, 0, s>>>(A, d_bricks3, nbricks3, list, d_fb3 + STAGE, d_fb3 + 4 + STAGE);
         DBM_LAUNCH_CHECK();
       }
       if (nnear3 > 0) {
@@ -1776,16 +1788,9 @@ struct SimImpl : SimBase {
         else k_gather<Q, D, P><<<dim3(nnear3, Q), 256, 0, s>>>(A, d_near3, nnear3, half);
         DBM_LAUNCH_CHECK();
       }
-      if (STAGE == 2 && fuse) {
-        if (nbricks3 > 0) {
-          const unsigned ge = (unsigned)std::min<int64_t>((int64_t)nbricks3 * 2, sm_count() * 4);
-          k_emit_bricks<Q><<<ge, 256, 0, s>>>(A, d_bricks3, half, nbricks3, d_fb3 + fb_head(), d_fb3 + STAGE);
-          DBM_LAUNCH_CHECK();
-        }
-        if (nnear3 > 0) {
-          k_emit_bricks<Q><<<nnear3, 256, 0, s>>>(A, d_near3, half, nnear3, nullptr, nullptr);
-          DBM_LAUNCH_CHECK();
-        }
+      if (STAGE == 2 && fuse && nnear3 > 0) {
+        k_emit_bricks<Q><<<nnear3, 256, 0, s>>>(A, d_near3, half, nnear3);
+        DBM_LAUNCH_CHECK();
       }
     }
     return DBM_OK;
@@ -2252,7 +2257,8 @@ struct SimImpl : SimBase {
     A.want_wexp = untiled ? 1 : 0;
     // fallback counts of the three stages, odd_f
     int* const fb = brick3_path() ? d_fb3 : d_fb;
-    A.odd_f = fb ? fb + 4 : nullptr;
+    A.odd_f = fb ? fb + kFbFlags : nullptr;
+    A.further = brick3_path() ? fb + 3 : nullptr;
     if (fb) DBM_CUDA(cudaMemsetAsync(fb, 0, (size_t)fb_head() * sizeof(int), s));
     // the gather's empty masks: written whole by one block per tile, else combined from zero
     bool dense = false, split = false, shared = false;  // shared: split if the device says so
@@ -2392,7 +2398,7 @@ struct SimImpl : SimBase {
     // the dense gather writes every control point's empty mask and, with displacements of one cell or
     // grid windows and unless the step keeps its intermediates, emits the points without an empty
     // direction itself
-    const int fuse = ((dense && !split && (near_ok || grid_w)) || brick3_path()) && !A.write_trace ? 1 : 0;
+    const int fuse = ((dense && !split && (near_ok || grid_w)) || (brick3_path() && brick3_y == 1)) && !A.write_trace ? 1 : 0;
     cpf_whole = !fuse;
     if (from_zero && !A.clear_emask) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (kTiles) {

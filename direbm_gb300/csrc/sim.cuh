@@ -132,6 +132,7 @@ struct Args {
   uint32_t* d_P;
   int clear_start, clear_emask;  // b.start cleared by the collision, emask by the placement
   int share_slots;  // (grid kernels) blocks that run at once, 0: one block per tile
+  int* further;     // (3D grid kernels) moments beyond one per cell, counted by the collision
   int* odd_f;      // (dense kernels) per instance, set by the collision: a density is negative or an f* not finite
   int write_trace;
 };

@@ -300,11 +300,11 @@ __device__ __forceinline__ void copy_async(float* dst, const float* src) { copy4
 __device__ __forceinline__ void copy_async(float2* dst, const float2* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
-// Copies direction k's plane of the region's items: `src` [mcap] of T, into buffer k & 1.
+// Copies one direction's plane of the region's items: `src` [mcap] of T, into buffer `buf`.
 template <class T, class SM>
-__device__ __forceinline__ void fetch_plane(const SM& S, int nmore, int k, const T* __restrict__ src) {
-  T* dst = S.template plane<T>(k & 1);
-  T* mdst = S.template mplane<T>(k & 1);
+__device__ __forceinline__ void fetch_plane(const SM& S, int nmore, int buf, const T* __restrict__ src) {
+  T* dst = S.template plane<T>(buf);
+  T* mdst = S.template mplane<T>(buf);
 #pragma unroll 2
   for (int ci = threadIdx.x; ci < kCells3; ci += kThreads3) {
     const int m = S.gi()[ci];
@@ -385,7 +385,7 @@ __device__ __forceinline__ bool thin_refine_brick(const Args<Q, 3, PF32>& A, con
 #pragma unroll 1
   for (int k = 0; k < Q; ++k) {
     fetch_wait();
-    if (k + 1 < Q) fetch_plane<float>(S, nmore, k + 1, A.wexp + (int64_t)(k + 1) * A.mcap);
+    if (k + 1 < Q) fetch_plane<float>(S, nmore, (k + 1) & 1, A.wexp + (int64_t)(k + 1) * A.mcap);
     const float cd[3] = {A.L.cdf[k][0], A.L.cdf[k][1], A.L.cdf[k][2]};
     const float base[3] = {cen[0] - cd[0], cen[1] - cd[1], cen[2] - cd[2]};
     Win3 w;
@@ -461,8 +461,8 @@ __device__ __forceinline__ bool thin_refine_brick(const Args<Q, 3, PF32>& A, con
 // ---- weights ------------------------------------------------------------------------------------
 
 template <int Q>
-__device__ __forceinline__ bool weights_brick(const Args<Q, 3, PF32>& A, const Brick& B, const InstK& I,
-                                              unsigned char* smem) {
+__device__ __forceinline__ bool weights_brick(const Args<Q, 3, PF32>& A, const Brick& B, const InstK& I, int share,
+                                              int shares, unsigned char* smem) {
   const Grid3Smem<1> S{smem};
   __shared__ GridOwn3 own;
   if (threadIdx.x == 0) *S.cnt() = own.n = own.taken = 0;
@@ -475,6 +475,7 @@ __device__ __forceinline__ bool weights_brick(const Args<Q, 3, PF32>& A, const B
   }
   bool has = m1 > m;
   for (int i = m + 1; i < m1 && !many; ++i) many = own.push(i, t) ? 0 : 1;
+  if (!__syncthreads_or(has)) return true;  // no moment in the brick
   if (!stage_grid3(I, B, A.b.start, A.b.off, A.ccap, S, many, [](int) { return 0.f; })) return false;
   const int nmore = *S.cnt();
   const float base0 = 768.f * __int_as_float(__float_as_int(A.R) & 0x7f800000);  // see GridWeightSum
@@ -489,7 +490,7 @@ __device__ __forceinline__ bool weights_brick(const Args<Q, 3, PF32>& A, const B
       for (int a = 0; a < 3; ++a) o[a] = A.a.off[(int64_t)a * A.mcap + m];
     }
 #pragma unroll 1
-    for (int k = 0; k < Q; ++k) {
+    for (int k = share; k < Q; k += shares) {
       const float cd[3] = {A.L.cdf[k][0], A.L.cdf[k][1], A.L.cdf[k][2]};
       const float base[3] = {rn_add(o[0], cd[0]), rn_add(o[1], cd[1]), rn_add(o[2], cd[2])};
       Win3 w;
@@ -530,8 +531,8 @@ __device__ __forceinline__ bool weights_brick(const Args<Q, 3, PF32>& A, const B
 // ---- gather -------------------------------------------------------------------------------------
 
 template <int Q>
-__device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Brick& B, const InstK& I, bool fuse,
-                                             unsigned char* smem) {
+__device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Brick& B, const InstK& I, int share,
+                                             int shares, bool fuse, unsigned char* smem) {
   const Grid3Smem<2> S{smem};
   __shared__ GridOwn3 own;
   if (threadIdx.x == 0) *S.cnt() = own.n = own.taken = 0;
@@ -544,6 +545,8 @@ __device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Br
   }
   bool has = j1 > j;
   for (int i = j + 1; i < j1 && !many; ++i) many = own.push(i, t) ? 0 : 1;
+  if (!__syncthreads_or(has)) return true;  // no control point in the brick
+  const bool split = shares > 1;
   const float* rho = A.a.rho;
   if (!stage_grid3(I, B, A.a.start, A.a.off, A.mcap, S, many, [&](int m) { return rho[m]; })) return false;
   const int nmore = *S.cnt();
@@ -561,11 +564,12 @@ __device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Br
     }
     uint32_t empty = 0;
     DF F[Q];
-    fetch_plane<float2>(S, nmore, 0, kvs);
+    int buf = 0;
+    fetch_plane<float2>(S, nmore, 0, kvs + (int64_t)share * A.mcap);
 #pragma unroll 1
-    for (int k = 0; k < Q; ++k) {
+    for (int k = share; k < Q; k += shares, buf ^= 1) {
       fetch_wait();
-      if (k + 1 < Q) fetch_plane<float2>(S, nmore, k + 1, kvs + (int64_t)(k + 1) * A.mcap);
+      if (k + shares < Q) fetch_plane<float2>(S, nmore, buf ^ 1, kvs + (int64_t)(k + shares) * A.mcap);
       const float cd[3] = {A.L.cdf[k][0], A.L.cdf[k][1], A.L.cdf[k][2]};
       const float base[3] = {p[0] - cd[0], p[1] - cd[1], p[2] - cd[2]};
       Win3 w;
@@ -575,8 +579,8 @@ __device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Br
                     [&](int a, float off, int jj) { return rn_add(off, canon_c<float>(jj, cd[a], p[a])); });
       GatherSum s;
       s.clear();
-      const float2* pk = S.plane<float2>(k & 1);
-      const float2* pm = S.mplane<float2>(k & 1);
+      const float2* pk = S.plane<float2>(buf);
+      const float2* pm = S.mplane<float2>(buf);
       window3<true>(S, nmore, has, c, w, [&](int a, int jj) { return canon_c<float>(jj, cd[a], p[a]); },
                     [&](float4 r, int i, int q, float cx, float cy, float cz) {
                       const float ex = rn_add(r.x, cx), ey = rn_add(r.y, cy), ez = rn_add(r.z, cz);
@@ -585,10 +589,18 @@ __device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Br
                       if (wgt > 0.f) kv = q < 0 ? pk[i] : pm[q];
                       s.add(__fmul_rn(wgt, kv.x), r.w, kv.y);
                     });
-      F[k] = gather_total(A.L.wf[k], A.L.wlo[k], s.hi, s.lo, s.sb);
-      if (F[k].hi < A.eps) empty |= 1u << k;
+      const DF Fk = gather_total(A.L.wf[k], A.L.wlo[k], s.hi, s.lo, s.sb);
+      if (Fk.hi < A.eps) empty |= 1u << k;
+      if (!split) {
+        F[k] = Fk;
+      } else if (has) {
+        A.cpfhi[(int64_t)k * A.ccap + j] = Fk.hi;
+        A.cpflo[(int64_t)k * A.ccap + j] = Fk.lo;
+      }
     }
-    if (has) {
+    if (split) {
+      if (has && empty) atomicOr(A.emask + j, empty);
+    } else if (has) {
       A.emask[j] = empty;
       if (fuse && !empty) {
         emit_full<Q>(A, j, F);
@@ -607,61 +619,101 @@ __device__ __forceinline__ bool gather_brick(const Args<Q, 3, PF32>& A, const Br
 
 // ---- kernels ----------------------------------------------------------------------------------------
 
-// STAGE: 0 thin + refine, 1 weights, 2 gather.
+// The moments beyond one per cell (noted by the collision) are more than 1 in 32: the region of a brick, 2744
+// cells, then holds about 86 of them where it is full, and bricks beyond the list of 128 are common.  Each
+// would be staged in vain and wait for the others to finish; the untiled kernels take all bricks instead (a
+// cluster of 20 k moments in 64^3 cells: 3006 -> 1494 us a step, 1466 by the untiled kernels' own launches).
+template <int Q>
+__device__ __forceinline__ bool crowded3(const Args<Q, 3, PF32>& A) {
+  return (int64_t)*A.further * 32 > (int64_t)*A.a.count;
+}
+
+// Called, not inlined: inline it takes registers from the grid kernel (64^3 cells: 411 -> 505 us).
+template <int Q>
+__device__ __noinline__ void thin_refine_apart(const Args<Q, 3, PF32>& A, uint32_t F, const InstK& I) {
+  thin_refine_cell<Q, 3, PF32>(A, F, I);
+}
+
+// STAGE: 0 thin + refine, 1 weights, 2 gather.  In boxes of few bricks gridDim.x / nbricks blocks share a
+// brick's directions in weights and gather; the gather then leaves its sums to the emit pass.  As many as run at
+// once: blocks beyond that, with nothing to do in a full box, set the others two on an SM (152 bricks:
+// weights 287 -> 365 us).  A brick that cannot be staged is thinned by the untiled code in the same
+// block (a cell per thread, as there); its weights and gather, where the untiled kernels spread the directions
+// over blocks, go to a second launch (k_brick3_fallback).
 template <int Q, int STAGE>
 __global__ void __launch_bounds__(kThreads3, 2) k_brick3(const __grid_constant__ Args<Q, 3, PF32> A,
                                                         const Brick* __restrict__ bricks, int nbricks,
                                                         int* fb_bricks, int* fb_count, int fuse) {
   extern __shared__ __align__(16) unsigned char smem[];
-  for (int bi = blockIdx.x; bi < nbricks; bi += gridDim.x) {
-    const Brick B = bricks[bi];
-    const InstK I = A.inst[B.inst];
-    bool ok;
-    if constexpr (STAGE == 0) ok = thin_refine_brick<Q>(A, B, I, smem);
-    else if constexpr (STAGE == 1) ok = weights_brick<Q>(A, B, I, smem);
-    // a negative density or an f that is not finite in the instance (noted by the collision): no brick
-    else ok = !A.odd_f[B.inst] && gather_brick<Q>(A, B, I, fuse != 0, smem);
-    if (!ok && threadIdx.x == 0) fb_bricks[atomicAdd(fb_count, 1)] = bi;
-    __syncthreads();
+  const int shares = gridDim.x / nbricks, bi = blockIdx.x / shares, share = blockIdx.x % shares;
+  if (crowded3(A)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *fb_count = nbricks;
+    return;
+  }
+  const Brick B = bricks[bi];
+  const InstK I = A.inst[B.inst];
+  bool ok;
+  if constexpr (STAGE == 0) ok = thin_refine_brick<Q>(A, B, I, smem);
+  else if constexpr (STAGE == 1) ok = weights_brick<Q>(A, B, I, share, shares, smem);
+  // a negative density or an f that is not finite in the instance (noted by the collision): no brick
+  else ok = !A.odd_f[B.inst] && gather_brick<Q>(A, B, I, share, shares, fuse != 0, smem);
+  if (ok || share > 0) return;
+  uint32_t g;
+  const bool valid = brick3_global(B, I, threadIdx.x, &g);
+  if constexpr (STAGE == 0) {
+    if (threadIdx.x == 0) atomicAdd(fb_count, 1);
+    if (valid) thin_refine_apart<Q>(A, g, I);
+  } else {
+    if (threadIdx.x == 0) fb_bricks[atomicAdd(fb_count, 1)] = bi;
+    if (STAGE == 2 && fuse && valid)
+      for (uint32_t j = A.b.start[g], j1 = A.b.start[g + 1]; j < j1; ++j) A.emask[j] = kEmitLater;
   }
 }
 
-// The untiled kernels on the deferred bricks, each as two bricks of 8 x 8 x 4 cells (thread t <-> cell t).
+// The untiled kernels on the deferred bricks (of a crowded state: on all), each as two bricks of 8 x 8 x 4
+// cells (thread t <-> cell t), direction by direction; blocks take the next unit as they finish one.  Registers
+// as those kernels (six blocks per SM).  5 % of 96^3 cells after a step: 29.1 -> 21.9 ms a step, 21.4 by the
+// untiled kernels' own launches.
 template <int Q, int STAGE>
-__global__ void __launch_bounds__(256) k_brick3_fallback(const __grid_constant__ Args<Q, 3, PF32> A,
-                                                        const Brick* __restrict__ bricks,
-                                                        const int* __restrict__ fb_bricks,
-                                                        const int* __restrict__ fb_count) {
+__global__ void __launch_bounds__(256, 6) k_brick3_fallback(const __grid_constant__ Args<Q, 3, PF32> A,
+                                                           const Brick* __restrict__ bricks, int nbricks,
+                                                           const int* __restrict__ fb_bricks,
+                                                           const int* __restrict__ fb_count, int* ticket) {
+  const bool all = crowded3(A);
+  if (STAGE == 0 && !all) return;
   const BrickGeo bg{kBrick3, kBrick3, kBrick3 / 2};
-  const int per = STAGE == 0 ? 2 : 2 * Q;
-  const int64_t n = (int64_t)*fb_count * per;
-  for (int64_t u = blockIdx.x; u < n; u += gridDim.x) {
-    const int e = (int)(u / per), r = (int)(u - (int64_t)e * per);
-    Brick B = bricks[fb_bricks[e]];
-    B.z0 += (r & 1) * (kBrick3 / 2);
+  const int n = 2 * (all ? nbricks : *fb_count);
+  const int64_t units = (int64_t)n * (STAGE == 0 ? 1 : Q);
+  __shared__ int s_next;
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_next = units > 0 ? atomicAdd(ticket, 1) : 0;
+    __syncthreads();
+    const int64_t u = s_next;
+    if (u >= units) return;
+    const int k = (int)(u / n), e = (int)(u - (int64_t)k * n);
+    Brick B = bricks[all ? e >> 1 : fb_bricks[e >> 1]];
+    B.z0 += (e & 1) * (kBrick3 / 2);
     const InstK I = A.inst[B.inst];
     uint32_t F;
     if (!brick_cell<3>(B, I, bg, threadIdx.x, &F)) continue;
     if constexpr (STAGE == 0) {
       thin_refine_cell<Q, 3, PF32>(A, F, I);
     } else if constexpr (STAGE == 1) {
-      for (uint32_t m = A.a.start[F], m1 = A.a.start[F + 1]; m < m1; ++m) weights_one<Q, 3, PF32>(A, m, r >> 1, F, I);
+      for (uint32_t m = A.a.start[F], m1 = A.a.start[F + 1]; m < m1; ++m) weights_one<Q, 3, PF32>(A, m, k, F, I);
     } else {
-      for (uint32_t j = A.b.start[F], j1 = A.b.start[F + 1]; j < j1; ++j) gather_one<Q, 3, PF32>(A, j, r >> 1, F, I);
+      for (uint32_t j = A.b.start[F], j1 = A.b.start[F + 1]; j < j1; ++j) gather_one<Q, 3, PF32>(A, j, k, F, I);
     }
   }
 }
 
-// Emits the control points without an empty direction of the bricks the untiled gather served (a list
-// of bricks of the given extent, or with fb_bricks the deferred ones of it).
+// Emits the control points without an empty direction of the bricks near an obstacle, which the untiled gather
+// served.
 template <int Q>
 __global__ void __launch_bounds__(256) k_emit_bricks(const __grid_constant__ Args<Q, 3, PF32> A,
-                                                    const Brick* __restrict__ bricks, BrickGeo bg, int nbricks,
-                                                    const int* __restrict__ fb_bricks, const int* __restrict__ fb_count) {
-  const int n = fb_bricks ? *fb_count * 2 : nbricks;
-  for (int u = blockIdx.x; u < n; u += gridDim.x) {
-    Brick B = bricks[fb_bricks ? fb_bricks[u >> 1] : u];
-    if (fb_bricks) B.z0 += (u & 1) * (kBrick3 / 2);
+                                                    const Brick* __restrict__ bricks, BrickGeo bg, int nbricks) {
+  for (int u = blockIdx.x; u < nbricks; u += gridDim.x) {
+    const Brick B = bricks[u];
     const InstK I = A.inst[B.inst];
     uint32_t F;
     if (!brick_cell<3>(B, I, bg, threadIdx.x, &F)) continue;

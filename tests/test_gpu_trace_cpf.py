@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("lattice,dims", [("D2Q9", (400, 390)), ("D3Q19", (16, 16, 16))])
+@pytest.mark.parametrize("lattice,dims", [("D2Q9", (400, 390)), ("D3Q19", (56, 48, 48))])
 @pytest.mark.parametrize("graphs", [True, False])
 def test_gathered_f_is_never_stale(lattice, dims, graphs):
     from direbm_gb300._lib import DbmError
