@@ -1834,6 +1834,9 @@ struct SimImpl : SimBase {
     return DBM_OK;
   }
   int brick_width() const override { return bgeo.bx; }
+  int window_path() const override {
+    return tiled_path() ? DBM_PATH_TILES : brick3_path() ? DBM_PATH_GRID3 : DBM_PATH_BRICKS;
+  }
 
   // Per-component buffers that only the untiled window kernels use: (1/sw, f*) pairs and exp(f*)
   // ([Q][mcap] each).  Allocated by the calls that make that path possible (creation in 3D, an
@@ -2977,6 +2980,12 @@ int dbm_sim_get_brick_width(dbm_sim* s, int32_t* brick_width) {
   SIM_CHECK(s);
   if (!brick_width) return DBM_ERR_INVALID;
   *brick_width = s->impl->brick_width();
+  return DBM_OK;
+}
+int dbm_sim_get_window_path(dbm_sim* s, int32_t* path) {
+  SIM_CHECK(s);
+  if (!path) return DBM_ERR_INVALID;
+  *path = s->impl->window_path();
   return DBM_OK;
 }
 int dbm_sim_get_tiling(dbm_sim* s, int32_t* tile_width, int32_t* persistent) {

@@ -360,6 +360,7 @@ struct SimBase {
   virtual int ensure_untiled() = 0;
   virtual int set_brick(int bx) = 0;
   virtual int brick_width() const = 0;
+  virtual int window_path() const = 0;  // DBM_PATH_*
   int kappa_soft = 0;  // soft-outer spawn threshold (0: off)
   int use_graphs = 1;
   int use_tiles = 1;

@@ -321,8 +321,8 @@ class Simulation:
         return int(w.value), bool(p.value)
 
     def set_tiling(self, tile_width: int | None = None, persistent: bool | None = None):
-        """Tiles of tile_width x 256/tile_width cells and/or persistent launches (2D only).  Results
-        are bit-identical for every setting; only the speed changes."""
+        """Tiles of tile_width x 256/tile_width cells and/or persistent launches (``window_path() ==
+        "tiles"``: 2D FP32 boxes).  Results are bit-identical for every setting; only the speed changes."""
         with torch.cuda.device(self.device):
             if tile_width is not None:
                 _lib.check(self.lib.dbm_sim_set_option(self._h, self.OPT_TILE_WIDTH, int(tile_width)), "set tile width")
@@ -346,6 +346,16 @@ class Simulation:
             _lib.check(self.lib.dbm_sim_set_option(self._h, self.OPT_DENSE_STENCIL, 1 if on else 0),
                        "set dense stencil")
 
+    WINDOW_PATHS = {1: "tiles", 2: "bricks", 3: "grid3"}
+
+    def window_path(self) -> str:
+        """The window kernels of the next step, and so which launch setting acts: "tiles" (2D FP32:
+        ``set_tiling``), "bricks" (the untiled kernels: ``set_brick_width``) or "grid3" (the 3D grid
+        kernels: neither)."""
+        p = ctypes.c_int32()
+        _lib.check(self.lib.dbm_sim_get_window_path(self._h, ctypes.byref(p)), "dbm_sim_get_window_path")
+        return self.WINDOW_PATHS[int(p.value)]
+
     def brick_width(self) -> int:
         """Cells along x of the 256-cell bricks the untiled window kernels give each block."""
         w = ctypes.c_int32()
@@ -354,8 +364,8 @@ class Simulation:
 
     def set_brick_width(self, width: int):
         """Bricks of width x (256 / width) cells (2D) or width x by x bz (3D) for the untiled window
-        kernels (3D, obstacles, the soft spawn, tiles off).  Results are bit-identical for every
-        width; only the speed changes."""
+        kernels (``window_path() == "bricks"``: FP64, 2D obstacles, the soft spawn, tiles off, 3D without
+        the grid kernels).  Results are bit-identical for every width; only the speed changes."""
         with torch.cuda.device(self.device):
             _lib.check(self.lib.dbm_sim_set_option(self._h, self.OPT_BRICK_WIDTH, int(width)), "set brick width")
 

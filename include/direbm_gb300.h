@@ -220,8 +220,8 @@ int dbm_sim_use_graphs(dbm_sim* sim, int32_t on);
  * r (none when that sum is below 1e-8).  Needs a moment capacity of 2 x cells (DBM_ERR_CAPACITY
  * otherwise); runs on the untiled kernels; the tape (dbm_tape_*) refuses a simulator with it on. */
 #define DBM_OPT_KAPPA_SOFT 5
-/* DBM_OPT_BRICK_WIDTH: the untiled window kernels (FP64, near obstacles, 3D radii without a grid kernel,
- * the soft spawn, tiles off) give
+/* DBM_OPT_BRICK_WIDTH: the untiled window kernels (DBM_PATH_BRICKS: FP64, 2D obstacles, the soft spawn, tiles
+ * or the 3D dense stencil off, 3D radii or displacements without a grid kernel) give
  * each block a brick of 256 cells, this many along x (a power of two, 4..32 in 3D, 8..64 in 2D;
  * default 8 in 3D, 16 in 2D); results do not depend on it.  direbm_gb300.autotune picks it. */
 #define DBM_OPT_BRICK_WIDTH 6
@@ -237,6 +237,13 @@ int dbm_sim_use_graphs(dbm_sim* sim, int32_t on);
  * window becomes a fixed 4 x 4 block of cells; other tiles take the row-segment loops in a second
  * launch (default 1).  Results are bit-identical either way. */
 #define DBM_OPT_DENSE_STENCIL 8
+/* Which window kernels the next step runs, and so which setting of the launch acts: the 2D tiled ones (tile
+ * width, persistence), the untiled ones (brick width), or the 3D grid kernels (neither: bricks of 8^3 cells,
+ * and of 8 x 8 x 4 near an obstacle). */
+#define DBM_PATH_TILES 1
+#define DBM_PATH_BRICKS 2
+#define DBM_PATH_GRID3 3
+int dbm_sim_get_window_path(dbm_sim* sim, int32_t* path);
 int dbm_sim_get_brick_width(dbm_sim* sim, int32_t* brick_width);
 int dbm_sim_set_option(dbm_sim* sim, int32_t option, int32_t value);
 int dbm_sim_get_tiling(dbm_sim* sim, int32_t* tile_width, int32_t* persistent);
