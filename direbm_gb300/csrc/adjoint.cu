@@ -1400,8 +1400,7 @@ struct TapeImpl : TapeBase, StepHook {
                     cudaStream_t s) {
     const size_t sm = list_smem_bytes<real, D, KIND>(256);
     if (!list_attr_set[KIND]) {
-      DBM_CUDA(cudaFuncSetAttribute((const void*)k_list<Q, D, P, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sm));
+      DBM_TRY(allow_smem((const void*)k_list<Q, D, P, KIND>, sm));
       list_attr_set[KIND] = true;
     }
     k_list<Q, D, P, KIND><<<g, 256, sm, s>>>(A, r, cp_of_cell, d_count + KIND);

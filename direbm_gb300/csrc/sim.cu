@@ -1707,7 +1707,7 @@ struct SimImpl : SimBase {
         }
       const void* k3[3] = {(const void*)k_brick3<Q, 0>, (const void*)k_brick3<Q, 1>, (const void*)k_brick3<Q, 2>};
       for (int i = 0; i < 3; ++i)
-        DBM_CUDA(cudaFuncSetAttribute(k3[i], cudaFuncAttributeMaxDynamicSharedMemorySize, grid3_layout(i).total));
+        DBM_TRY(allow_smem(k3[i], grid3_layout(i).total));
       brick3_ok = true;
       DBM_TRY(make_bricks3());
     }
@@ -1988,12 +1988,9 @@ struct SimImpl : SimBase {
       DBM_CUDA(cudaMemset(d_fb, 0, ((size_t)ntiles + fb_head()) * sizeof(int)));
     }
     if constexpr (kTiles) {
-      DBM_CUDA(cudaFuncSetAttribute((const void*)k_thin_refine_t<Q, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sm_refine));
-      DBM_CUDA(cudaFuncSetAttribute((const void*)k_weights_t<Q, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sm_weights));
-      DBM_CUDA(cudaFuncSetAttribute((const void*)k_gather_t<Q, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sm_gather));
+      DBM_TRY(allow_smem((const void*)k_thin_refine_t<Q, P>, sm_refine));
+      DBM_TRY(allow_smem((const void*)k_weights_t<Q, P>, sm_weights));
+      DBM_TRY(allow_smem((const void*)k_gather_t<Q, P>, sm_gather));
       int nb[3] = {1, 1, 1};
       DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[0], k_thin_refine_t<Q, P>, 256, sm_refine));
       DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb[1], k_weights_t<Q, P>, 256, sm_weights));
@@ -2008,7 +2005,7 @@ struct SimImpl : SimBase {
         });
         int slots = 1 << 30;
         for (int i = 0; i < 3; ++i) {
-          DBM_CUDA(cudaFuncSetAttribute(kg[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_grid[i]));
+          DBM_TRY(allow_smem(kg[i], sm_grid[i]));
           int nbd = 1;
           DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kg[i], 256, sm_grid[i]));
           pgrid_grid[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
@@ -2020,18 +2017,15 @@ struct SimImpl : SimBase {
         args.share_slots = grid_y > 1 ? slots : 0;
       }
       if (shift_ok) {
-        DBM_CUDA(cudaFuncSetAttribute((const void*)k_gather_ts<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sm_gather_s));
+        DBM_TRY(allow_smem((const void*)k_gather_ts<Q>, sm_gather_s));
         int nbs = 1;
         DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbs, k_gather_ts<Q>, 256, sm_gather_s));
         pgrid_s = std::max(1, std::min(ntiles, std::max(nbs, 1) * sm_count()));
-        DBM_CUDA(cudaFuncSetAttribute((const void*)k_thin_refine_t<Q, P, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
+        DBM_TRY(allow_smem((const void*)k_thin_refine_t<Q, P, true>, sm_refine));
         int nbr = 1;
         DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbr, k_thin_refine_t<Q, P, true>, 256, sm_refine));
         pgrid_rs = std::max(1, std::min(ntiles, std::max(nbr, 1) * sm_count()));
-        DBM_CUDA(cudaFuncSetAttribute((const void*)k_weights_t<Q, P, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_weights));
+        DBM_TRY(allow_smem((const void*)k_weights_t<Q, P, true>, sm_weights));
         int nbw = 1;
         DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbw, k_weights_t<Q, P, true>, 256, sm_weights));
         pgrid_ws = std::max(1, std::min(ntiles, std::max(nbw, 1) * sm_count()));
@@ -2042,7 +2036,7 @@ struct SimImpl : SimBase {
           kds[2] = (const void*)k_gather_ds<Q, tx.value, false>;
         });
         for (int i = 0; i < 3; ++i) {
-          DBM_CUDA(cudaFuncSetAttribute(kds[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
+          DBM_TRY(allow_smem(kds[i], sm_ds[i]));
           int nbd = 1;
           DBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbd, kds[i], 256, sm_ds[i]));
           pgrid_ds[i] = std::max(1, std::min(ntiles, std::max(nbd, 1) * sm_count()));
@@ -2050,17 +2044,14 @@ struct SimImpl : SimBase {
           if constexpr (Q == 9) {
             if (i > 0 && near_ok && geo.tx == 32 && ntiles * 3 <= std::max(nbd, 1) * sm_count()) {
               split_ds[i] = 3;
-              DBM_CUDA(cudaFuncSetAttribute(i == 1 ? (const void*)k_weights_ds<Q, 32, true> : (const void*)k_gather_ds<Q, 32, true>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_ds[i]));
+              DBM_TRY(allow_smem(i == 1 ? (const void*)k_weights_ds<Q, 32, true> : (const void*)k_gather_ds<Q, 32, true>,
+                                 sm_ds[i]));
             }
           }
         }
-        DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 0>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_refine));
-        DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 1>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_weights));
-        DBM_CUDA(cudaFuncSetAttribute((const void*)k_dense_fallback<Q, 2>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_gather_s));
+        DBM_TRY(allow_smem((const void*)k_dense_fallback<Q, 0>, sm_refine));
+        DBM_TRY(allow_smem((const void*)k_dense_fallback<Q, 1>, sm_weights));
+        DBM_TRY(allow_smem((const void*)k_dense_fallback<Q, 2>, sm_gather_s));
       }
     }
     tiled = true;

@@ -10,6 +10,7 @@
 // round-to-nearest operations, so each (m, k) makes the same integer decisions everywhere.
 #pragma once
 
+#include <mutex>
 #include <type_traits>
 
 #include "lattice.cuh"
@@ -312,6 +313,18 @@ __device__ __forceinline__ bool inside_sphere(const InstK& I, const int (&S)[3],
     d2 = a == 0 ? e2 : __dadd_rn(d2, e2);
   }
   return d2 < I.obs_r2;
+}
+
+// Lets launches of `kernel` take `bytes` of dynamic shared memory.  The limit belongs to the kernel, not to a
+// simulator, so it only grows: one set up for less may not take away what another's launches need.
+inline int allow_smem(const void* kernel, size_t bytes) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  cudaFuncAttributes a;
+  DBM_CUDA(cudaFuncGetAttributes(&a, kernel));
+  if ((size_t)a.maxDynamicSharedSizeBytes < bytes)
+    DBM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return DBM_OK;
 }
 
 // Called around one step by SimBase::step_hooked.  `before` sees the input state (args->a, not
