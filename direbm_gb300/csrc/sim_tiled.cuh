@@ -200,7 +200,7 @@ __device__ __forceinline__ void thin_refine_body(const Args<Q, 2, P>& A, const I
   uint32_t cnt = 0;
   real cen[3] = {0, 0, 0};
   if (valid) {
-      CSum csum[2];
+    CSum csum[2];
 #pragma unroll 1
     for (int k = 0; k < Q; ++k) {
       const real cdx = A.L.template cd_as<real>(k, 0), cdy = A.L.template cd_as<real>(k, 1);
