@@ -1459,8 +1459,9 @@ struct SimImpl : SimBase {
   cudaGraphExec_t graph_tr[2] = {nullptr, nullptr};  // the same step writing every intermediate
   unsigned long long graph_kernels = 0, graph_tr_kernels = 0;
   int trace_on = 0;
-  // the last step's gather left all its sums in memory (DBM_TRACE_CPF); graph_cpf: a captured step does
-  bool cpf_whole = true, graph_cpf = true;
+  // the last step's gather left all its sums in memory (DBM_TRACE_CPF); graph_cpf: a captured step does;
+  // cpf_redo: its inputs are still there (regather)
+  bool cpf_whole = true, graph_cpf = true, cpf_redo = false;
   // shared-memory tiling (2D)
   bool tiled = false;
   Tile2* d_tiles = nullptr;
@@ -2184,6 +2185,7 @@ struct SimImpl : SimBase {
     if (m > 0 && (!inst_of || !pos || !fin)) { set_last_error("set_state: null input"); return DBM_ERR_INVALID; }
     cur = 0;
     ++version;
+    cpf_redo = false;
     const bool presorted = (flags & kLoadPresorted) != 0;
     if (flags & kLoadF32)
       return import_sorted_states<float>(m, s, inst_of, (const float*)pos, (const float*)fin, presorted);
@@ -2237,6 +2239,7 @@ struct SimImpl : SimBase {
   bool grid_path() const { return grid_w != 0 && use_dense && tiled_path(); }
 
   int launch_step(cudaStream_t s, int upto) {
+    cpf_redo = false;
     bind();
     Args<Q, D, P>& A = args;
     mark(0, s);
@@ -2394,6 +2397,7 @@ struct SimImpl : SimBase {
     // direction itself
     const int fuse = ((dense && !split && (near_ok || grid_w)) || (brick3_path() && brick3_y == 1)) && !A.write_trace ? 1 : 0;
     cpf_whole = !fuse;
+    cpf_redo = true;
     if (from_zero && !A.clear_emask) DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
     if constexpr (kTiles) {
       if (tiled_path()) {
@@ -2464,6 +2468,7 @@ struct SimImpl : SimBase {
         }
         DBM_CUDA(cudaGraphLaunch(graph[cur], own));
         cpf_whole = graph_cpf;
+        cpf_redo = true;
         count_launch(graph_kernels);
       } else {
         DBM_TRY(launch_step(own, 99));
@@ -2616,6 +2621,7 @@ struct SimImpl : SimBase {
   }
 
   int push_instances() {
+    cpf_redo = false;
     DBM_CUDA(cudaStreamSynchronize(own));  // no step may still read the table
     DBM_CUDA(cudaMemcpy(dinst, inst_h.data(), sizeof(InstK) * inst_h.size(), cudaMemcpyHostToDevice));
     int any = 0;
@@ -2684,6 +2690,7 @@ struct SimImpl : SimBase {
     DBM_CUDA(cudaStreamWaitEvent(own, ev_in, 0));
     cur = 0;
     ++version;
+    cpf_redo = false;
     bind();
     StateP<P>& S = st[0];
     const char* p = (const char*)src + snap_align(sizeof(SnapHeader));
@@ -2744,6 +2751,29 @@ struct SimImpl : SimBase {
     return DBM_OK;
   }
 
+  // The last step's gathered f, when its gather emitted most points from registers: once more, by the row-segment
+  // or untiled kernel (the same bits), from the step's collided moments and weights.
+  int regather(cudaStream_t s) {
+    if constexpr (std::is_same<P, PF32>::value) {
+      if (cpf_whole) return DBM_OK;
+      if (!cpf_redo) {
+        set_last_error("trace: the last step's gathered f is gone (the state or an instance was set since)");
+        return DBM_ERR_STATE;
+      }
+      cur ^= 1;
+      bind();
+      Args<Q, D, P> A = args;
+      cur ^= 1;
+      bind();
+      DBM_CUDA(cudaMemsetAsync(A.emask, 0, (size_t)ccap * 4, s));
+      if constexpr (kTiles) k_gather_t<Q, P><<<ntiles, 256, sm_gather, s>>>(A, d_tiles, geo, ntiles);
+      else k_gather<Q, D, P><<<dim3(nbricks, Q), 256, 0, s>>>(A, d_bricks, nbricks, bgeo);
+      DBM_LAUNCH_CHECK();
+      cpf_whole = true;
+    }
+    return DBM_OK;
+  }
+
   int trace(int what, void* dst, int64_t nbytes, int64_t* needed, cudaStream_t s) override {
     const void* src = nullptr;
     int64_t sz = 0;
@@ -2764,14 +2794,11 @@ struct SimImpl : SimBase {
       case DBM_TRACE_CPF:
         if constexpr (std::is_same<P, PF64>::value) { src = A.cpf64; sz = (int64_t)Q * ccap * 8; }
         else {
-          if (!cpf_whole) {  // the gather emitted most points from registers: what is there is of older steps
-            set_last_error("trace: a plain step keeps no gathered f (dbm_sim_step_partial does)");
-            return DBM_ERR_STATE;
-          }
           sz = (int64_t)2 * Q * ccap * 4;
           if (needed) *needed = sz;
           if (dst) {
             if (nbytes < sz) { set_last_error("trace: destination too small"); return DBM_ERR_INVALID; }
+            DBM_TRY(regather(s));
             DBM_CUDA(cudaMemcpyAsync(dst, A.cpfhi, (size_t)Q * ccap * 4, cudaMemcpyDeviceToDevice, s));
             DBM_CUDA(cudaMemcpyAsync((char*)dst + (size_t)Q * ccap * 4, A.cpflo, (size_t)Q * ccap * 4,
                                      cudaMemcpyDeviceToDevice, s));

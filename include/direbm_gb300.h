@@ -351,8 +351,9 @@ int dbm_tape_export(dbm_tape* tape, int32_t index, int32_t what, void* d_dst, in
 #define DBM_TRACE_FINAL_OFF 6  /* real[D][ncells] refined CP offset */
 #define DBM_TRACE_SORTED 7     /* u32[2][P]     sorted (cell, origin cell) pairs */
 #define DBM_TRACE_SW 8         /* real[Q][Mcap] 1/sw per component, 0 if dropped (FP32DEV: float) */
-#define DBM_TRACE_CPF 9        /* FP64: double[Q][cap]; FP32DEV: float[2][Q][cap] (hi, lo), of
-                                  dbm_sim_step_partial; DBM_ERR_STATE after a step that kept it in registers */
+#define DBM_TRACE_CPF 9        /* FP64: double[Q][cap]; FP32DEV: float[2][Q][cap] (hi, lo), of the last step
+                                  (gathered again if that kept it in registers; DBM_ERR_STATE if the state or
+                                  an instance was set since) */
 #define DBM_TRACE_EMPTY 10     /* u32[cap]      empty-direction mask per CP */
 #define DBM_TRACE_FSTAR 11     /* collided f of the input moments, layout of the state */
 #define DBM_TRACE_COUNTS 12    /* u32[2]: M (moments in), P (control points) */

@@ -1,5 +1,5 @@
-"""The gathered f as a trace buffer: right after a partial step, refused (not stale) after a step whose gather
-emitted from registers."""
+"""The gathered f as a trace buffer: the last step's, also where that step's gather emitted from registers, and
+never an older step's."""
 
 import numpy as np
 import pytest
@@ -27,16 +27,33 @@ def test_gathered_f_is_never_stale(lattice, dims, graphs):
         s.set_state(None, x, f)
         return s
 
+    def gathered(s):
+        p = s.count()
+        return s.trace("cpf").cpu().numpy().view(np.float32).reshape(2, get(lattice).Q, s.capacity)[:, :, :p]
+
     a, b = sim(), sim(dense=False)
-    for _ in range(2):  # the second from a recorded graph
-        a.step(1)
-        b.step(1)
-        with pytest.raises(DbmError):
-            a.trace("cpf")
+    for n in (1, 1, 2):  # the later ones from recorded graphs
+        a.step(n)
+        b.step(n)
+        np.testing.assert_array_equal(gathered(a), gathered(b))
+        np.testing.assert_array_equal(gathered(a), gathered(b))
+        empty = [s.trace("empty").cpu().numpy().view(np.uint32)[: s.count()] for s in (a, b)]
+        np.testing.assert_array_equal(*empty)
+    a.set_state(None, x, f)  # without a step, there is no gathered f of this state
+    a.step(1)
+    a.set_state(None, x, f)
+    with pytest.raises(DbmError):
+        a.trace("cpf")
+    a.step(1)
+    b.set_state(None, x, f)
+    b.step(1)
+    for i, (u, v) in enumerate(zip(a.state_numpy(), b.state_numpy())):
+        np.testing.assert_array_equal(u, v)
+    np.testing.assert_array_equal(gathered(a), gathered(b))
+    for s in (a, b):
+        s.step(1)  # goes on from the state that the reading left alone
+    for u, v in zip(a.state_numpy(), b.state_numpy()):
+        np.testing.assert_array_equal(u, v)
     for s in (a, b):
         s.step_partial(6)
-    p = a.count()
-    read = [s.trace("cpf").cpu().numpy().view(np.float32).reshape(2, get(lattice).Q, s.capacity)[:, :, :p] for s in (a, b)]
-    np.testing.assert_array_equal(*read)
-    a.step(1)  # intermediates are kept from the first partial step on
-    a.trace("cpf")
+    np.testing.assert_array_equal(gathered(a), gathered(b))
