@@ -1779,7 +1779,8 @@ struct SimImpl : SimBase {
         const unsigned grid = (unsigned)nbricks3 * (STAGE == 0 ? 1 : brick3_y);
         k_brick3<Q, STAGE><<<grid, kThreads3, smem, s>>>(A, d_bricks3, nbricks3, list, d_fb3 + STAGE, fuse);
         DBM_LAUNCH_CHECK();
-        const unsigned gf = (unsigned)std::min<int64_t>((int64_t)nbricks3 * (STAGE == 0 ? 2 : 2 * Q), sm_count() * 6);
+        const int64_t units = 2 * (int64_t)nbricks3;
+        const unsigned gf = (unsigned)(STAGE == 0 ? units : std::min<int64_t>(units * Q, sm_count() * 6));
         k_brick3_fallback<Q, STAGE><<<gf, 256, 0, s>>>(A, d_bricks3, nbricks3, list, d_fb3 + STAGE, d_fb3 + 4 + STAGE);
         DBM_LAUNCH_CHECK();
       }

@@ -671,9 +671,11 @@ __global__ void __launch_bounds__(kThreads3, 2) k_brick3(const __grid_constant__
 }
 
 // The untiled kernels on the deferred bricks (of a crowded state: on all), each as two bricks of 8 x 8 x 4
-// cells (thread t <-> cell t), direction by direction; blocks take the next unit as they finish one.  Registers
-// as those kernels (six blocks per SM).  5 % of 96^3 cells after a step: 29.1 -> 21.9 ms a step, 21.4 by the
-// untiled kernels' own launches.
+// cells (thread t <-> cell t), registers as those kernels (six blocks per SM).  Thin + refine, whose blocks do
+// little but for crowded states, has one per unit (handed out one by one: 423 -> 519 us in a cluster of 16 k
+// moments in 64^3 cells); weights and gather, with Q times as many units, take the next as they finish one,
+// direction by direction.  5 % of 96^3 cells after a step: 29.1 -> 21.9 ms a step, 21.4 by the untiled kernels'
+// own launches.
 template <int Q, int STAGE>
 __global__ void __launch_bounds__(256, 6) k_brick3_fallback(const __grid_constant__ Args<Q, 3, PF32> A,
                                                            const Brick* __restrict__ bricks, int nbricks,
@@ -682,8 +684,16 @@ __global__ void __launch_bounds__(256, 6) k_brick3_fallback(const __grid_constan
   const bool all = crowded3(A);
   if (STAGE == 0 && !all) return;
   const BrickGeo bg{kBrick3, kBrick3, kBrick3 / 2};
+  if constexpr (STAGE == 0) {
+    Brick B = bricks[blockIdx.x >> 1];
+    B.z0 += (int)(blockIdx.x & 1) * (kBrick3 / 2);
+    const InstK I = A.inst[B.inst];
+    uint32_t F;
+    if (brick_cell<3>(B, I, bg, threadIdx.x, &F)) thin_refine_cell<Q, 3, PF32>(A, F, I);
+    return;
+  }
   const int n = 2 * (all ? nbricks : *fb_count);
-  const int64_t units = (int64_t)n * (STAGE == 0 ? 1 : Q);
+  const int64_t units = (int64_t)n * Q;
   __shared__ int s_next;
   for (;;) {
     __syncthreads();
@@ -697,9 +707,7 @@ __global__ void __launch_bounds__(256, 6) k_brick3_fallback(const __grid_constan
     const InstK I = A.inst[B.inst];
     uint32_t F;
     if (!brick_cell<3>(B, I, bg, threadIdx.x, &F)) continue;
-    if constexpr (STAGE == 0) {
-      thin_refine_cell<Q, 3, PF32>(A, F, I);
-    } else if constexpr (STAGE == 1) {
+    if constexpr (STAGE == 1) {
       for (uint32_t m = A.a.start[F], m1 = A.a.start[F + 1]; m < m1; ++m) weights_one<Q, 3, PF32>(A, m, k, F, I);
     } else {
       for (uint32_t j = A.b.start[F], j1 = A.b.start[F + 1]; j < j1; ++j) gather_one<Q, 3, PF32>(A, j, k, F, I);
